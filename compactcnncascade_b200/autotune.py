@@ -7,13 +7,13 @@ The knobs (include/ccnn_inspect.h, ccnn_schedule):
   frame_slots          frames in flight, each with its own stream, buffers and captured graph
   window_ctas_per_sm   resident blocks per SM of the persistent stage-2/3 window kernel (5, 6: builds
                        with 48 and 40 registers a thread)
-  front_blocks_per_sm  register budget of the stage-1 front kernel (3: 80 registers, 4: 64)
-  back_blocks_per_sm   register budget of the stage-1 back kernel (3: 80 registers, 4: 64)
+  front_blocks_per_sm  register budget of the stage-1 front kernel (3: 5 blocks of 128 threads a SM, 4: 6)
+  back_blocks_per_sm   register budget of the stage-1 back kernel (3: 5 blocks of 128 threads a SM, 4: 6)
   batch_frames         frames per batched graph (0: every frame its own graph; 1: the same with the
                        pyramid and stage 1 of all levels in one persistent launch); the batched form
                        runs the pyramid and stage 1 of a whole group in one persistent launch
-  batch_blocks_per_sm  resident blocks per SM of that persistent kernel (its grid; 4: 64 registers,
-                       1-3: 80; fewer leave SMs to other frames' kernels)
+  batch_blocks_per_sm  how much of a SM that persistent kernel fills (its grid: twice this many blocks of 128
+                       threads a SM, at most the 5 that fit; fewer leave SMs to other frames' kernels)
 
 The search is coordinate descent from the defaults: each knob in turn takes the value that times
 fastest with the others held, for two passes (a full product of the knobs would be 960 timings).

@@ -94,23 +94,24 @@ __device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
 }
 
 // Correctly rounded IEEE reciprocals of two values in [1, 2^126): the hardware approximation
-// (rcp.approx, within about an ulp) refined by two Newton-Raphson steps with fused residuals,
-// e = 1 - d*y, y' = y + y*e (Markstein's FMA iteration). For every float of that range the result
-// equals __frcp_rn bit for bit (compared exhaustively on B200, ccnn_check_reciprocal). Outside it
-// (subnormal results, infinity, NaN) both lanes take __frcp_rn.
+// (rcp.approx, within about an ulp) refined by one Newton-Raphson step with fused residuals,
+// e = 1 - d*y, y' = y + y*e (Markstein's FMA iteration; a second step changes no value). For every float
+// of that range the result equals __frcp_rn bit for bit (compared exhaustively on B200,
+// ccnn_check_reciprocal). Outside it (subnormal results, infinity, NaN) both lanes take __frcp_rn.
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+// -1 times the operand: both lanes of nd in (-2^126, -1], or NaN
+__device__ __forceinline__ f2_t f2_rcp_neg(f2_t nd) {
+    const f2_t y = f2_pack(rcp_approx(-f2_lo(nd)), rcp_approx(-f2_hi(nd)));
+    return f2_fma(y, f2_fma(nd, y, f2_pack(1.f, 1.f)), y);
+}
 __device__ __forceinline__ f2_t f2_rcp(f2_t d) {
     const float d0 = f2_lo(d), d1 = f2_hi(d);
     if (!(d0 >= 1.f && d0 < 0x1p126f && d1 >= 1.f && d1 < 0x1p126f)) return f2_pack(__frcp_rn(d0), __frcp_rn(d1));
-    const f2_t one = f2_pack(1.f, 1.f);
-    const f2_t nd = f2_pack(-d0, -d1);
-    f2_t y = f2_pack(rcp_approx(d0), rcp_approx(d1));
-    y = f2_fma(y, f2_fma(nd, y, one), y);
-    return f2_fma(y, f2_fma(nd, y, one), y);
+    return f2_rcp_neg(f2_pack(-d0, -d1));
 }
 
 // Two independent lanes of tanh_rational. The reciprocal 1/den is the correctly rounded IEEE
@@ -125,6 +126,26 @@ __device__ __forceinline__ f2_t tanh_rational2(f2_t c, f2_t nz) {
     const f2_t r = f2_rcp(den);  // den >= 1 (or NaN)
     const f2_t sgn = f2_pack(lo < 0.f ? -1.f : 1.f, hi < 0.f ? -1.f : 1.f);
     return f2_mul(sgn, f2_sub(one, r), nz);
+}
+
+// 0.5 * tanh_rational(c) + 0.5 of two lanes as fma(+-0.5, 1 - 1/den, 0.5), the sign c's: halving is exact,
+// so the single rounding of the fma is that of the reference's sum, and the sign costs no multiply
+// (sgn(-0) is +1 in the reference, but 1 - 1/den is +0 there, and 0.5 +- 0 is 0.5). The denominator is
+// clamped at 2^125 (from 2^25 on 1 - 1/den is 1), NaN kept, so the reciprocal needs no range check.
+__device__ __forceinline__ float neg_clamp_den(float den) {  // max(-den, -2^125), NaN if den is
+    float r;
+    asm("{ .reg .f32 t; neg.f32 t, %1; max.NaN.f32 %0, t, 0fFE000000; }" : "=f"(r) : "f"(den));
+    return r;
+}
+__device__ __forceinline__ f2_t tanh_half2(f2_t c, f2_t nz, f2_t half) {
+    const f2_t a = f2_pack(1.41645f, 1.41645f);
+    const float lo = f2_lo(c), hi = f2_hi(c);
+    const f2_t ac1 = f2_pack(fadd(1.f, fabsf(lo)), fadd(1.f, fabsf(hi)));
+    const f2_t c2 = f2_mul(c, c, nz);
+    const f2_t c4 = f2_mul(f2_mul(f2_mul(f2_mul(a, c, nz), c, nz), c, nz), c, nz);
+    const f2_t den = f2_add(f2_add(ac1, c2), c4);
+    const f2_t r = f2_rcp_neg(f2_pack(neg_clamp_den(f2_lo(den)), neg_clamp_den(f2_hi(den))));
+    return f2_fma(f2_pack(copysignf(0.5f, lo), copysignf(0.5f, hi)), f2_sub(f2_pack(1.f, 1.f), r), half);
 }
 
 // Two lanes of lrelu_bn; p = {b, w1, w2, bn_b}, each a (lane 0, lane 1) pair.
@@ -173,17 +194,29 @@ using Stage2W = NetWeights<6, 12, 24, 4, 4, 3, 3, 7, 8, 84, 4, 4>;
 // cnn4face3_cntk.bin: 36x40 window, 6/12/24 maps, 4x4 / 3x3 / 7(w)x8(h), hidden 34 = 17 x 2
 using Stage3W = NetWeights<6, 12, 24, 4, 4, 3, 3, 7, 8, 34, 8, 2>;
 
-// Stage-1 parameters duplicated (v, v) for the back kernel, which runs every operation of the L3
-// maps, the hidden layer and the output neuron on two vertically adjacent response pixels at once.
-struct Stage1Dup {
-    float2 k3d[Stage1W::kM3][Stage1W::kK3W * Stage1W::kK3H];
-    float2 a3d[Stage1W::kM3][4];
-    float2 hwd[Stage1W::kHL][Stage1W::kConn];
-    float2 hbd[Stage1W::kHL];
-    float2 htwd[Stage1W::kGroups];
-    float2 hbnwd[Stage1W::kHS], hbnbd[Stage1W::kHS];
-    float2 owd[Stage1W::kHL];
-    float2 obd, otwd, afd;
+// Stage-1 parameters of layers 2 and 3, the hidden layer and the output for the back kernel, which runs
+// every operation on two response (or pooled) pixels at once: each value duplicated (v, v), in the order
+// the kernel walks them and in whole 16-byte groups, so that one constant load brings two of them (a
+// constant load a value was 15 % of the kernel's instructions).
+struct alignas(16) Stage1Back {
+    struct alignas(16) L2Map {
+        float2 k[10];  // the 9 taps (the 10th is unused)
+        float2 a[4];   // b, w2a, w2b, bn
+    } l2[Stage1W::kM2];
+    struct alignas(16) L3Map {
+        float2 k[Stage1W::kK3W * Stage1W::kK3H];
+        float2 a[4];
+    } l3[Stage1W::kM3];
+    struct alignas(16) Neuron {
+        float2 b, w[Stage1W::kConn], o;  // hidden bias and weights, the output neuron's weight
+    } hid[Stage1W::kHL];
+    float2 htw[Stage1W::kGroups + 1];    // per-group tanh slope (and one unused)
+    struct alignas(16) Slot {
+        float2 w, b;                     // batch normalisation of the group's neuron t
+    } hbn[Stage1W::kHS];
+    float2 ob, otw, af, negzero;
+    int half_out;                        // af == 0: the output is 0.5 * tanh + 0.5
+    int pad[3];
 };
 
 // cnn4landmarks_cntk.bin (facial analysis): 49x51 window, 24/48/96 maps, 4x4 / 3x3 / 10(w)x11(h),
@@ -226,7 +259,9 @@ struct LevelDesc {
     int p1w, p1h;        // L1 pooled size: (w-3)>>1, (h-3)>>1
     int p2w, p2h;        // L2 pooled size: (p1w-2)>>1, (p1h-2)>>1
     int ow, oh;          // response map: p2w-3, p2h-4
-    int s1_pitch;        // floats per row of each S1 plane
+    int s1_pitch;        // floats per row of each S1 plane (a multiple of 32): a row holds its even columns,
+                         // then from s1_pitch / 2 its odd ones (the back kernel's 2x2 pooling walks columns in
+                         // steps of two)
     long long s1_off;    // offset of this level's S1 planes in the S1 arena (floats)
     long long s1_plane;  // floats per S1 plane
     long long resp_off;  // offset of this level's response map (dense, pitch ow)

@@ -800,7 +800,7 @@ ccnn_status Detector::enqueue_kernels(Slot& s, const Plan& p) {
         build_batch_queue(&Q, 1, p.n_levels, (int)p.chunks.size(), p.k1_tiles, p.k2_tiles, cfg_.thr1);
         CCNN_CUDA(cudaMemsetAsync(s.d_sync1, 0, sizeof(int) * (2 + kBatchStages), s.st));
         CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, s.d_sync1, s.d_sync1 + 1 + kBatchStages,
-                                      sm_count_ * stage1_batch_blocks_per_sm(batch_bpsm_), s.st, batch_bpsm_));
+                                      sm_count_ * stage1_batch_blocks_per_sm(batch_bpsm_), s.st));
         CCNN_CUDA(cudaMemcpyAsync(s.h_nfaces + 1, s.d_sync1 + 1 + kBatchStages, sizeof(int), cudaMemcpyDeviceToHost, s.st));
     } else {
         // the legacy network reads stored level images; the CNTK front kernel resamples its tiles from
@@ -1469,7 +1469,7 @@ ccnn_status Detector::profile(int iters, float* ms, int n_ms) {
             CCNN_CUDA(cudaMemsetAsync(s.d_sync1, 0, sizeof(int) * (2 + kBatchStages), s.st));
             if (!p.chunks.empty()) CCNN_CUDA(cudaMemsetAsync(s.d_counts, 0, sizeof(int) * p.chunks.size(), s.st));
             CCNN_CUDA(cudaEventRecord(ev[0], s.st));
-            CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, s.d_sync1, s.d_sync1 + 1 + kBatchStages, grid, s.st, batch_bpsm_));
+            CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, s.d_sync1, s.d_sync1 + 1 + kBatchStages, grid, s.st));
             CCNN_CUDA(cudaEventRecord(ev[1], s.st));
             CCNN_CUDA(cudaEventSynchronize(ev[1]));
             float m = 0.f;
@@ -1679,7 +1679,7 @@ ccnn_status Detector::enqueue_batch_kernels(BatchCtx& c, const Plan& p, int B) {
     const int grid = sm_count_ * stage1_batch_blocks_per_sm(batch_bpsm_);
     int* sync = c.d_sync;
     int* err = c.d_sync + 1 + kBatchStages * B;
-    CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, sync, err, grid, st, batch_bpsm_));
+    CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, sync, err, grid, st));
     CCNN_CUDA(launch_cand_write_batch(p.d_chunks, (int)p.chunks.size(), p.d_levels, F, C, B, cfg_.thr1, (int)cand_cap_, st));
     if (detect_enabled_) CCNN_CUDA(launch_window_batch(*wn_, WB, gpitch, p.gw, p.gh, p.d_levels, cfg_, window_grid_, st, window_ctas_per_sm_));
     CCNN_CUDA(launch_replay_batch(c.d_rargs, B, st));

@@ -5,19 +5,24 @@
 // add/add2 (:916-950), conv_3x3 (:36-91), conv_5x4 (:158-187), lrelu_bn (:623-645),
 // mulCN_add_tanhW (:646-672), mulC/mulC1_add (:952-984), tanhW (:673-690).
 //
-// front: one CTA per 32x16 tile of pooled L1 pixels of one level. The CTA resamples its (67 x 35)
-//        input tile straight from the gray frame (the pyramid is never stored; a stored image is read
-//        instead where the caller gives one; with the learned gate each warp resamples only the 7
-//        rows of its own two pooled rows and runs on its own), runs the 4x4 conv + folded
+// front: one CTA of 128 threads per 32x16 tile of pooled L1 pixels of one level. The CTA resamples its
+//        (67 x 35) input tile straight from the gray frame (the pyramid is never stored; a stored image is
+//        read instead where the caller gives one; with the learned gate each warp resamples only the 7
+//        rows of a strip of two pooled rows and runs on its own), runs the 4x4 conv + folded
 //        BN/LReLU + 2x2 max for the 4 L1 maps and writes the 4 neighbour-map sums that L2 consumes
-//        (S1 arena).
-// back:  one CTA per 32x16 tile of response pixels. It stages the S1 tile (4 x 42 x 72) one map at a
-//        time through two shared-memory buffers (asynchronous copies of the next map overlap the
-//        current one's compute), computes the 8 pooled L2 maps and their sums on the 35 x 20 halo
-//        tile, then every thread finishes two vertically adjacent response pixels: the 16 L3 maps
-//        (4w x 5h), the 52 hidden neurons and the output neuron.
-// Both kernels come in two register budgets (3 or 4 resident 256-thread blocks per SM), chosen per
-// workload by the schedule (Stage1Sched).
+//        (S1 arena). Bound by the fp32 pipe (65 % busy; about 87 % is what these packed chains reach
+//        alone) and the latency of the gray samples: 1.09 ms for the 83 levels of a 3840x2160 frame at
+//        scale 1.05 (1.30 with 256-thread blocks and 25 % more instructions: the row references once a
+//        tile instead of once a sample, both gray rows of a sample as one packed chain), 39.8 us for the
+//        13 of a 1080p frame (43.3).
+// back:  one CTA per 32x16 tile of response pixels (128 threads with two pixel pairs a thread, 256 with
+//        one). It takes the S1 tile (4 x 42 x 72) map by map through two shared-memory buffers
+//        (asynchronous copies), computes the pooled L2 maps of each and the sums they complete on the
+//        35 x 20 halo tile, then the 16 L3 maps (4w x 5h), the 52 hidden neurons and the output sum as far
+//        as those reach. Bound by the fp32 pipe (65 % busy): 1.35 ms for the 83 levels (1.64 when a thread
+//        packed two vertical neighbours, whose operands had to be paired in registers, with two
+//        reciprocal steps and twice the constant loads a pixel), 53 us for the 13 (61).
+// Both kernels come in two register budgets, chosen per workload by the schedule (Stage1Sched).
 // Packed f32x2 instructions run two identical chains of IEEE operations at once (two pixels, or
 // two maps that read the same input), so every value still sees the reference's roundings.
 // Every tile of every level is one block of the same grid; a block finds its level by binary
@@ -32,18 +37,18 @@ constexpr int kInW = 2 * kK1TileX + 3;  // 67
 constexpr int kInH = 2 * kK1TileY + 3;  // 35
 constexpr int kInWh = (kInW + 1) / 2;   // 34 columns of each parity
 
+constexpr int kFrontThreads = 128;
+constexpr int kStrips = kK1TileY / 2;  // a strip: two pooled rows, 32 columns
+constexpr int kStripRows = 7;          // input rows of a strip
+
 // One input sample of the front tile: row r, column c (tile coordinates) = value v. Row r is
 // stored next to row r+2 as a packed pair (a thread computes two vertically adjacent pooled
 // pixels, whose windows are 2 rows apart), and columns are split by parity so that the stride-2
 // column walk of a warp is conflict-free.
 struct FrontTile {
     float2 p[kInH - 2][2][kInWh];
-    float tail[2][kInW];  // the last two rows have no partner below
     __device__ __forceinline__ void put(int r, int c, float v) {
-        if (r < kInH - 2)
-            p[r][c & 1][c >> 1].x = v;
-        else
-            tail[r - (kInH - 2)][c] = v;
+        if (r < kInH - 2) p[r][c & 1][c >> 1].x = v;
         if (r >= 2) p[r - 2][c & 1][c >> 1].y = v;
     }
 };
@@ -51,9 +56,7 @@ struct FrontTile {
 // Loads the (67 x 35) input tile of a front CTA from its level image. Rows that start 16-byte
 // aligned with a pitch of whole float4 groups are read as 17 float4 per row (columns past the
 // image width hold zeros or the caller's own padding; no stored pixel depends on them), other
-// images one float at a time. kCoherent: the image was written earlier in the same launch (read
-// through L2, never the read-only path).
-template <bool kCoherent>
+// images one float at a time.
 __device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __restrict__ img, const LevelDesc& L, int ix0, int iy0) {
     if (L.img_vec) {
         constexpr int kV = (kInW + 3) / 4;  // 17
@@ -63,7 +66,7 @@ __device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __res
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (y < L.h && x < L.img_pitch) {
                 const float4* src = reinterpret_cast<const float4*>(img + (long long)y * L.img_pitch + x);
-                v = kCoherent ? __ldcg(src) : __ldg(src);
+                v = __ldg(src);
             }
             T.put(r, 4 * c4, v.x);
             T.put(r, 4 * c4 + 1, v.y);
@@ -75,86 +78,127 @@ __device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __res
             const int r = i / kInW, c = i - r * kInW;
             const int x = ix0 + c, y = iy0 + r;
             const float* src = img + (long long)y * L.img_pitch + x;
-            T.put(r, c, (x < L.w && y < L.h) ? (kCoherent ? __ldcg(src) : __ldg(src)) : 0.f);
+            T.put(r, c, (x < L.w && y < L.h) ? (__ldg(src)) : 0.f);
         }
     }
 }
 
-// The input rows of one warp of a gated front tile: warp w computes pooled rows 2w and 2w + 1 from
-// tile rows 4w .. 4w + 6, held here as local rows 0..6, row r next to row r + 2 (columns split by
-// parity, as in FrontTile). Rows 4w + 4 .. 4w + 6 are also the next warp's first three; each warp
-// resamples its own copy, so no block barrier separates resampling and compute.
-struct FrontWarpRows {
-    float2 p[5][2][kInWh];
+// The input rows of one strip of a gated front tile, held as local rows 0..6, row r next to row r + 2
+// (columns split by parity, as in FrontTile). Rows 4..6 are also the next strip's first three; each
+// warp resamples its own copy, so no block barrier separates resampling and compute.
+struct FrontStripRows {
+    float2 p[kStripRows - 2][2][kInWh];
     __device__ __forceinline__ void put(int r, int c, float v) {
-        if (r <= 4) p[r][c & 1][c >> 1].x = v;
+        if (r < kStripRows - 2) p[r][c & 1][c >> 1].x = v;
         if (r >= 2) p[r - 2][c & 1][c >> 1].y = v;
     }
 };
 
-struct FrontSmem {
-    union {
-        FrontTile T;                    // the block's whole input tile (full scan, or a stored level image)
-        FrontWarpRows w[kK1TileY / 2];  // each warp's own input rows (gated scan from the gray frame)
-    };
+// Where a level row is sampled: the gray row's offset (floats) and, for bilinear levels, the row weights
+// (of the row and of the one below).
+struct alignas(16) RowRef {
+    uint32_t off;
+    float pad;
+    float2 cf;
 };
 
-// level pixel (x, y) = tile (c, r) from its column sample sx
-__device__ __forceinline__ float resample_px(const GrayRef& G, const LevelDesc& L, const AxisSample& sx, int x, int y) {
-    if (x >= L.w || y >= L.h) return 0.f;
-    if (L.mode == 0) return __ldg(G.p + (size_t)y * G.pitch + x);
+struct FrontSmem {
+    union {
+        FrontTile T;                               // the block's whole input tile (full scan, or a stored level image)
+        FrontStripRows w[kFrontThreads / 32];      // each warp's own input rows (gated scan from the gray frame)
+    };
+    RowRef rows[kInH];                             // of the tile's rows, or kStripRows a warp
+};
+
+__device__ __forceinline__ RowRef row_ref(const GrayRef& G, const LevelDesc& L, int y) {
+    RowRef r{};
+    if (L.mode == 0) {
+        r.off = (uint32_t)min(y, G.h - 1) * (uint32_t)G.pitch;
+        return r;
+    }
     const AxisSample sy = sample_row(y, L.scly, G.h);
-    if (L.mode == 1) return __ldg(G.p + (size_t)sy.idx * G.pitch + sx.idx);
     uint32_t py = sy.idx;
-    if (py + 1 >= (uint32_t)G.h) py--;  // bilinear keeps a row below
-    const float* r0 = G.p + (size_t)py * G.pitch + sx.idx;
-    const float top = fadd(fmul(__ldg(r0), sx.c), fmul(__ldg(r0 + 1), sx.f));
-    const float bot = fadd(fmul(__ldg(r0 + G.pitch), sx.c), fmul(__ldg(r0 + G.pitch + 1), sx.f));
-    return fadd(fmul(top, sy.c), fmul(bot, sy.f));
+    if (L.mode == 2 && py + 1 >= (uint32_t)G.h) py--;  // bilinear keeps a row below
+    r.off = py * (uint32_t)G.pitch;
+    r.cf = make_float2(sy.c, sy.f);
+    return r;
 }
 
-// Front-tile input straight from the gray frame: every level pixel resampled the way the pyramid
-// kernel writes it (copy, nearest neighbour, or bilinear on the 12-bit fixed-point steps;
-// RunCPUDetect, cnn_detector_v3.cpp:2090-2104, with ImageResizer, image_resize.cpp:46-122, 393-541),
-// so the level image is never stored. Pixels outside the level read as 0, like the zero columns past
-// a stored level image's width. The gray frame was written by an earlier launch (read-only path).
-//
-// The whole (67 x 35) tile by the block (the full scan: every warp computes, so no row is resampled
-// twice): thread (g, c) takes tile column c < 64 (its column sample in registers) and rows g, g + 4,
-// ... of it, so a warp reads 32 neighbouring columns of the same gray rows; columns 64-66 follow, one
-// sample a thread.
-__device__ __forceinline__ void resample_front_tile(FrontTile& T, const GrayRef& G, const LevelDesc& L, int ix0, int iy0) {
-    static_assert(kInW == 67 && kInH == 35, "64 + 3 columns, 35 rows in 4 row groups");
-    {
-        const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-        const AxisSample sx = sample_col(ix0 + c, L.sclx, G.w);
-#pragma unroll
-        for (int k = 0; k < (kInH + 3) / 4; ++k) {
-            const int r = g + 4 * k;
-            if (r < kInH) T.put(r, c, resample_px(G, L, sx, ix0 + c, iy0 + r));
-        }
+// A level column: the gray column and, for bilinear levels, the column weights as pairs (both gray rows
+// of a sample run packed).
+struct ColRef {
+    uint32_t x;
+    f2_t c, f;
+};
+__device__ __forceinline__ ColRef col_ref(const GrayRef& G, const LevelDesc& L, int x) {
+    ColRef r;
+    if (L.mode == 0) {
+        r.x = (uint32_t)min(x, G.w - 1);
+        r.c = r.f = 0ull;
+        return r;
     }
-    if (threadIdx.x < 3 * kInH) {
+    const AxisSample sx = sample_col(x, L.sclx, G.w);
+    r.x = sx.idx;
+    r.c = f2_dup(sx.c);
+    r.f = f2_dup(sx.f);
+    return r;
+}
+
+// Level pixels straight from the gray frame, resampled the way the pyramid kernel writes them (copy,
+// nearest neighbour, or bilinear on the 12-bit fixed-point steps; RunCPUDetect,
+// cnn_detector_v3.cpp:2090-2104, with ImageResizer, image_resize.cpp:46-122, 393-541), so the level image
+// is never stored. The gray frame was written by an earlier launch (read-only path). Samples past the
+// level's last row or column read the frame's own last ones: no stored pooled pixel depends on them.
+// kBilinear: (p0 * cx + p1 * fx) of the two gray rows as one packed chain, then top * cy + bot * fy.
+template <bool kBilinear>
+__device__ __forceinline__ float resample_px(const GrayRef& G, const RowRef& row, const ColRef& col, f2_t nz) {
+    const float* p = G.p + (row.off + col.x);
+    if (!kBilinear) return __ldg(p);
+    const float* q = p + G.pitch;
+    const f2_t l = f2_pack(__ldg(p), __ldg(q)), r = f2_pack(__ldg(p + 1), __ldg(q + 1));
+    const f2_t h = f2_mul(f2_add(f2_mul(l, col.c, nz), f2_mul(r, col.f, nz)), f2_ld(row.cf), nz);
+    return fadd(f2_lo(h), f2_hi(h));
+}
+
+// The whole (67 x 35) tile by the block (the full scan: every strip is computed, so no row is resampled
+// twice): warp w takes rows w, w + 4, ... with the row's reference broadcast from shared memory, lane l
+// columns l and l + 32 with theirs in registers; columns 64-66 follow, one sample a thread. `rows`: tile
+// rows that lie in the level.
+template <bool kBilinear>
+__device__ __forceinline__ void resample_front_tile(FrontSmem& S, const GrayRef& G, const LevelDesc& L, int ix0, int rows, f2_t nz) {
+    static_assert(kInW == 67 && 3 * kInH <= kFrontThreads, "64 + 3 columns, one edge sample a thread");
+    constexpr int kWarps = kFrontThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const ColRef ca = col_ref(G, L, ix0 + lane), cb = col_ref(G, L, ix0 + lane + 32);
+#pragma unroll 3
+    for (int r = warp; r < rows; r += kWarps) {
+        const RowRef row = S.rows[r];
+        const float va = resample_px<kBilinear>(G, row, ca, nz), vb = resample_px<kBilinear>(G, row, cb, nz);
+        S.T.put(r, lane, va);
+        S.T.put(r, lane + 32, vb);
+    }
+    if (threadIdx.x < 3 * rows) {
         const int c = 64 + threadIdx.x % 3, r = threadIdx.x / 3;
-        T.put(r, c, resample_px(G, L, sample_col(ix0 + c, L.sclx, G.w), ix0 + c, iy0 + r));
+        S.T.put(r, c, resample_px<kBilinear>(G, S.rows[r], col_ref(G, L, ix0 + c), nz));
     }
 }
 
-// One warp's 7 input rows from tile row y0 on (the gated scan, where warps run on their own): lane l
-// takes tile columns l and l + 32 (their column samples in registers); columns 64-66 of the rows
-// follow, one sample a lane.
-__device__ __forceinline__ void resample_warp_rows(FrontWarpRows& R, const GrayRef& G, const LevelDesc& L, int ix0, int y0, int lane) {
-    const AxisSample sa = sample_col(ix0 + lane, L.sclx, G.w), sb = sample_col(ix0 + lane + 32, L.sclx, G.w);
+// One strip's 7 input rows (the gated scan, where warps run on their own): lane l takes columns l and
+// l + 32; columns 64-66 of the rows follow, one sample a lane.
+template <bool kBilinear>
+__device__ __forceinline__ void resample_strip(FrontStripRows& R, const RowRef* rows, const GrayRef& G, const LevelDesc& L, int ix0, f2_t nz) {
+    const int lane = threadIdx.x & 31;
+    const ColRef ca = col_ref(G, L, ix0 + lane), cb = col_ref(G, L, ix0 + lane + 32);
 #pragma unroll
-    for (int r = 0; r < 7; ++r) {
-        const float va = resample_px(G, L, sa, ix0 + lane, y0 + r);
-        const float vb = resample_px(G, L, sb, ix0 + lane + 32, y0 + r);
+    for (int r = 0; r < kStripRows; ++r) {
+        const RowRef row = rows[r];
+        const float va = resample_px<kBilinear>(G, row, ca, nz), vb = resample_px<kBilinear>(G, row, cb, nz);
         R.put(r, lane, va);
         R.put(r, lane + 32, vb);
     }
-    if (lane < 21) {
+    if (lane < 3 * kStripRows) {
         const int c = 64 + lane % 3, r = lane / 3;
-        R.put(r, c, resample_px(G, L, sample_col(ix0 + c, L.sclx, G.w), ix0 + c, y0 + r));
+        R.put(r, c, resample_px<kBilinear>(G, rows[r], col_ref(G, L, ix0 + c), nz));
     }
 }
 
@@ -180,157 +224,183 @@ __device__ __forceinline__ bool gate_live(const GateCells& cells, const LevelDes
 }
 
 // Front tile t of level L: its (67 x 35) level-image tile in shared memory (resampled from the gray
-// frame G when kFromGray, by the block, or with the gate by each warp for its own 7 rows; else read
-// from the stored level images limg by the block), then the 4x4 conv + folded
-// BN/LReLU + 2x2 max of the 4 L1 maps for 32 x 16 pooled pixels (two vertically adjacent pixels a
-// thread) and the 4 neighbour-map sums written to the S1 arena. kCoherent: a stored level image was
-// written earlier in the same launch (read through L2, not the read-only path).
-// cells (the learned gate, optional): a warp whose S1 strip (2 rows x 32 columns) feeds no live
-// response pixel writes nothing. S1 row y feeds pooled-L2 rows ceil((y - 3) / 2) .. y / 2 (a 3x3
-// conv at the 2x2 pool positions), and L2 row Y feeds response rows Y - 4 .. Y (the 4-wide, 5-tall L3
-// kernel); columns alike with the 4-wide kernel. The back kernel computes exactly the live pixels'
-// inputs, so a skipped strip is never read for a value that is kept.
-template <bool kFromGray, bool kCoherent>
+// frame G when kFromGray, by the block, or with the gate by each warp for the 7 rows of a strip; else read
+// from the stored level images limg by the block), then the 4x4 conv + folded BN/LReLU + 2x2 max of the 4
+// L1 maps for 32 x 16 pooled pixels, a warp a strip of 2 x 32 (two vertically adjacent pixels a thread), and
+// the 4 neighbour-map sums written to the S1 arena.
+// cells (the learned gate, optional): a strip that feeds no live response pixel is not computed. S1 row y
+// feeds pooled-L2 rows ceil((y - 3) / 2) .. y / 2 (a 3x3 conv at the 2x2 pool positions), and L2 row Y
+// feeds response rows Y - 4 .. Y (the 4-wide, 5-tall L3 kernel); columns alike with the 4-wide kernel. The
+// back kernel computes exactly the live pixels' inputs, so a skipped strip is never read for a value that
+// is kept.
+template <bool kFromGray>
 __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const LevelDesc& L, int t, const float* __restrict__ limg,
                                            const GrayRef& G, float* __restrict__ s1, const GateCells& cells) {
+    constexpr int kWarps = kFrontThreads / 32;
     const int px0 = (t % L.k1_tiles_x) * kK1TileX;
     const int py0 = (t / L.k1_tiles_x) * kK1TileY;
     const int ix0 = 2 * px0, iy0 = 2 * py0;
-
     const int qx = threadIdx.x & (kK1TileX - 1);
-    const int qy = (threadIdx.x >> 5) * 2;
-    // with the gate: whether the warp has a live pixel downstream (warp w computes pooled rows 2w, 2w + 1)
-    auto warp_live = [&]() {
-        const int ya = py0 + qy, yb = ya + 1, xa = px0, xb = px0 + kK1TileX - 1;
+    const int warp = threadIdx.x >> 5;
+    const int strips = min(kStrips, (L.p1h - py0 + 1) >> 1);  // those with pooled rows inside the level
+    const f2_t nz = f2_ld(W.negzero);
+    // with the gate: whether strip s has a live pixel downstream
+    auto strip_live = [&](int s) {
+        const int ya = py0 + 2 * s, yb = ya + 1, xa = px0, xb = px0 + kK1TileX - 1;
         return gate_live(cells, L, ((xa - 3 + 1) >> 1) - 3, xb >> 1, ((ya - 3 + 1) >> 1) - 4, yb >> 1);
     };
-    const float2(*In)[2][kInWh];  // In[r] = (input row 2qy + r, row 2qy + r + 2), r = 0..4
-    if (kFromGray && gate_gating(cells)) {
-        // with the gate every warp runs on its own: its liveness, its 7 input rows, its two pooled rows
-        // (the rows a live warp shares with a dead neighbour are not resampled twice over the tile, and
-        // no warp waits for the block)
-        int lv = 0;
-        if ((threadIdx.x & 31) == 0) lv = warp_live() ? 1 : 0;
-        if (!__shfl_sync(0xffffffffu, lv, 0)) return;  // no live response pixel downstream of this warp
-        FrontWarpRows& R = S.w[threadIdx.x >> 5];
-        resample_warp_rows(R, G, L, ix0, iy0 + 2 * qy, threadIdx.x & 31);
-        __syncwarp();
-        In = R.p;
-    } else if (kFromGray) {
-        // the full scan: the block resamples the tile once
-        resample_front_tile(S.T, G, L, ix0, iy0);
-        __syncthreads();
-        In = &S.T.p[2 * qy];
-    } else {
-        uint32_t live = 0xffu;
-        if (gate_gating(cells)) {
-            __shared__ int s_flive[kK1TileY / 2];
-            if ((threadIdx.x & 31) == 0) s_flive[threadIdx.x >> 5] = warp_live() ? 1 : 0;
-            __syncthreads();
-            live = 0u;
+    // the four L1 maps of strip s from its input rows In[r] = (row 4s + r, row 4s + r + 2), r = 0..4, and
+    // their neighbour sums into the arena
+    auto strip = [&](int s, const float2(*In)[2][kInWh]) {
+        // pr[r][c] = (input row 4s + r, row 4s + r + 2) at column 2qx + c: the windows of both pixels
+        f2_t pr[5][5];
 #pragma unroll
-            for (int w = 0; w < kK1TileY / 2; ++w)
-                if (s_flive[w]) live |= 1u << w;
-        }
-        load_front_tile<kCoherent>(S.T, limg + L.img_off, L, ix0, iy0);
-        __syncthreads();
-        if (!((live >> (threadIdx.x >> 5)) & 1u)) return;  // no live response pixel downstream of this warp
-        In = &S.T.p[2 * qy];
-    }
-    const f2_t nz = f2_ld(W.negzero);
-    // pr[r][c] = (input row 2qy+r, row 2qy+r+2) at column 2qx+c: the windows of both pixels
-    f2_t pr[5][5];
+        for (int r = 0; r < 5; ++r)
 #pragma unroll
-    for (int r = 0; r < 5; ++r)
-#pragma unroll
-        for (int c = 0; c < 5; ++c) pr[r][c] = *reinterpret_cast<const f2_t*>(&In[r][c & 1][qx + (c >> 1)]);
+            for (int c = 0; c < 5; ++c) pr[r][c] = f2_ld(In[r][c & 1][qx + (c >> 1)]);
 
-    // packed over the two pixels (lo = row qy, hi = row qy + 1)
-    f2_t P[4];
+        // packed over the two pixels (lo = row 2s, hi = row 2s + 1)
+        f2_t P[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        f2_t cv[4];
+        for (int m = 0; m < 4; ++m) {
+            f2_t cv[4];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const int dy = d >> 1, dx = d & 1;
-            f2_t acc = f2_mul(pr[dy][dx], f2_ld(W.k1d[m][0]), nz);
+            for (int d = 0; d < 4; ++d) {
+                const int dy = d >> 1, dx = d & 1;
+                f2_t acc = f2_mul(pr[dy][dx], f2_ld(W.k1d[m][0]), nz);
 #pragma unroll
-            for (int k = 1; k < 16; ++k) acc = f2_add(acc, f2_mul(pr[dy + (k >> 2)][dx + (k & 3)], f2_ld(W.k1d[m][k]), nz));
-            cv[d] = lrelu_bn2(acc, W.a1d[m], nz);
+                for (int k = 1; k < 16; ++k) acc = f2_add(acc, f2_mul(pr[dy + (k >> 2)][dx + (k & 3)], f2_ld(W.k1d[m][k]), nz));
+                cv[d] = lrelu_bn2(acc, W.a1d[m], nz);
+            }
+            P[m] = f2_max4(cv[0], cv[1], cv[2], cv[3]);
         }
-        P[m] = f2_max4(cv[0], cv[1], cv[2], cv[3]);
+        // neighbour-map sums consumed by L2 (add/add2 of the reference)
+        const f2_t s01 = f2_add(P[0], P[1]);
+        const f2_t o[4] = {s01, f2_add(s01, P[2]), f2_add(f2_add(P[1], P[2]), P[3]), f2_add(P[2], P[3])};
+        const int gx = px0 + qx, gy = py0 + 2 * s;
+        if (gx < L.p1w) {
+            // a row holds its even columns, then its odd ones
+            float* out = s1 + L.s1_off + (long long)gy * L.s1_pitch + ((gx & 1) ? L.s1_pitch >> 1 : 0) + (gx >> 1);
+            const bool two = gy + 1 < L.p1h;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                out[0] = f2_lo(o[k]);
+                if (two) out[L.s1_pitch] = f2_hi(o[k]);
+                out += L.s1_plane;
+            }
+        }
+    };
+    if (kFromGray && gate_gating(cells)) {
+        // with the gate every warp runs on its own: its strips' liveness, their 7 input rows, their two
+        // pooled rows (the rows a live strip shares with a dead neighbour are not resampled twice over the
+        // tile, and no warp waits for the block)
+        RowRef* rows = &S.rows[warp * kStripRows];
+        static_assert(kWarps * kStripRows <= kInH, "a row table a warp");
+        const int lane = threadIdx.x & 31;
+#pragma unroll 1
+        for (int s = warp; s < strips; s += kWarps) {
+            int lv = 0;
+            if (lane == 0) lv = strip_live(s) ? 1 : 0;
+            if (!__shfl_sync(0xffffffffu, lv, 0)) continue;  // no live response pixel downstream of this strip
+            __syncwarp();
+            if (lane < kStripRows) rows[lane] = row_ref(G, L, iy0 + 4 * s + lane);
+            __syncwarp();
+            if (L.mode == 2)
+                resample_strip<true>(S.w[warp], rows, G, L, ix0, nz);
+            else
+                resample_strip<false>(S.w[warp], rows, G, L, ix0, nz);
+            __syncwarp();
+            strip(s, S.w[warp].p);
+        }
+        return;
     }
-    // neighbour-map sums consumed by L2 (add/add2 of the reference)
-    const f2_t s01 = f2_add(P[0], P[1]);
-    const f2_t o[4] = {s01, f2_add(s01, P[2]), f2_add(f2_add(P[1], P[2]), P[3]), f2_add(P[2], P[3])};
-    const int gx = px0 + qx, gy = py0 + qy;
-    if (gx < L.p1w) {
-        float* out = s1 + L.s1_off + (long long)gy * L.s1_pitch + gx;
-        if (gy < L.p1h) {
+    uint32_t live = (1u << strips) - 1u;
+    if (kFromGray) {
+        // the full scan: the block resamples the tile once
+        if (threadIdx.x < kInH) S.rows[threadIdx.x] = row_ref(G, L, iy0 + threadIdx.x);
+        __syncthreads();
+        const int rows = 4 * strips + 3;
+        if (L.mode == 2)
+            resample_front_tile<true>(S, G, L, ix0, rows, nz);
+        else
+            resample_front_tile<false>(S, G, L, ix0, rows, nz);
+    } else {
+        if (gate_gating(cells)) {
+            __shared__ int s_flive[kStrips];
+            if (threadIdx.x < kStrips) s_flive[threadIdx.x] = strip_live(threadIdx.x) ? 1 : 0;
+            __syncthreads();
 #pragma unroll
-            for (int k = 0; k < 4; ++k) out[k * L.s1_plane] = f2_lo(o[k]);
+            for (int s = 0; s < kStrips; ++s)
+                if (!s_flive[s]) live &= ~(1u << s);
         }
-        if (gy + 1 < L.p1h) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) out[k * L.s1_plane + L.s1_pitch] = f2_hi(o[k]);
-        }
+        load_front_tile(S.T, limg + L.img_off, L, ix0, iy0);
     }
+    __syncthreads();
+#pragma unroll 1
+    for (int s = warp; s < strips; s += kWarps)
+        if ((live >> s) & 1u) strip(s, &S.T.p[4 * s]);  // a strip without a live pixel downstream writes nothing
 }
 
 
 // kFromGray: level tiles resampled from the gray frame G (the detection path), else read from the
 // stored level images limg (a caller's own level image)
 template <bool kFromGray, int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) stage1_front_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ LevelTable LT,
+__global__ void __launch_bounds__(kFrontThreads, kMinBlocks) stage1_front_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ LevelTable LT,
                                                               const float* __restrict__ limg, const GrayRef G, float* __restrict__ s1,
                                                               const uint8_t* __restrict__ front_on, const GateCells cells) {
     __shared__ FrontSmem S;
     const int g = LT.first + blockIdx.x;
     if (front_on && !front_on[g]) return;  // gated off: no back tile reads this one
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k1_base>(LT, g)];
-    front_tile<kFromGray, false>(W, S, L, g - L.k1_base, limg, G, s1, cells);
+    front_tile<kFromGray>(W, S, L, g - L.k1_base, limg, G, s1, cells);
 }
 
 constexpr int kP2TW = kK2TileX + 3;   // 35 pooled L2 columns (halo 3)
 constexpr int kP2TH = kK2TileY + 4;   // 20 pooled L2 rows (halo 4)
 constexpr int kS1TW = 2 * kP2TW + 2;  // 72
 constexpr int kS1TH = 2 * kP2TH + 2;  // 42
-constexpr int kS2P = kP2TW + 1;       // 36: ts2 row pitch
+constexpr int kHalfX = kK2TileX / 2;  // 16: pixels x and x + 16 of a row run as a packed pair
+constexpr int kS2P = kHalfX + 3;      // 19 pairs a row of pooled L2 pixels (columns 16-18 are in two pairs)
 
 struct BackSmem {
-    float s1[2][kS1TH][kS1TW];    // two S1 maps of the tile, row-major: map k in s1[k & 1] (double buffer)
-    float s2[8][kP2TH][kS2P];     // the 8 neighbour sums of the pooled L2 maps
+    // two S1 maps of the tile (map k in s1[k & 1]), each row its even columns, then its odd ones: a warp's
+    // 2x2-pooling windows read consecutive words
+    float s1[2][kS1TH][2][kS1TW / 2];
+    // the neighbour sums of the pooled L2 maps that this S1 map completes (at most three), column x next to
+    // column x + 16: the taps of a thread's response pixels load as packed pairs
+    float2 s2[3][kP2TH][kS2P];
 };
-constexpr int kBackSmemBytes = (int)sizeof(BackSmem);  // 47,232 B: four blocks fit a SM
-constexpr int kP2Px = kP2TW * kP2TH;                    // 700 pooled L2 pixels of a tile
-constexpr int kP2Passes = (kP2Px + 255) / 256;          // 3
+constexpr int kP2Units = kS2P * kP2TH;  // 380 pairs of pooled L2 pixels of a tile
 
-// Pooled L2 pixel k of a tile: the 32 x 20 block first (a warp takes 32 consecutive columns of one
-// row, so its shared-memory reads and writes are conflict-free), then the 3 x 20 right edge.
-__device__ __forceinline__ void p2_pixel(int p, int* x, int* y) {
-    if (p < 32 * kP2TH) {
-        *x = p & 31;
-        *y = p >> 5;
+// Pooled L2 pair k of a tile: the 16 x 20 block first (a warp takes two rows of 16 pairs: no bank
+// conflicts), then the 3 x 20 right edge.
+__device__ __forceinline__ void p2_unit(int p, int* x, int* y) {
+    if (p < kHalfX * kP2TH) {
+        *x = p & (kHalfX - 1);
+        *y = p / kHalfX;
     } else {
-        const int q = p - 32 * kP2TH;
-        *x = 32 + q % 3;
+        const int q = p - kHalfX * kP2TH;
+        *x = kHalfX + q % 3;
         *y = q / 3;
     }
 }
 
-// S1 map k of a back tile into S.s1[k & 1] by asynchronous 16-byte copies (cp.async through L2, one
-// commit group); columns past the plane pitch and rows past p1h are zero-filled (no valid response
-// pixel depends on them). The copies land while the block computes on the other buffer.
+// S1 map k of a back tile into shared memory by asynchronous 16-byte copies (cp.async through L2);
+// columns past the plane pitch and rows past p1h are zero-filled (no valid response pixel depends on
+// them).
+template <int kThreads>
 __device__ __forceinline__ void load_back_map_async(BackSmem& S, const float* __restrict__ s1, const LevelDesc& L, int sx0, int sy0, int k) {
     const float* base = s1 + L.s1_off + (long long)k * L.s1_plane;
-    constexpr int kV = kS1TW / 4;
-    float* buf = &S.s1[k & 1][0][0];
-    for (int i = threadIdx.x; i < kS1TH * kV; i += blockDim.x) {
-        const int rr = i / kV, c4 = i - rr * kV;
-        const int x = sx0 + 4 * c4, y = sy0 + rr;
-        const bool in = y < L.p1h && x < L.s1_pitch;  // x and the pitch are multiples of 4: the whole vector is in the row
-        const float* src = in ? base + (long long)y * L.s1_pitch + x : base;
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + rr * kS1TW + 4 * c4);
+    constexpr int kV = kS1TW / 8;  // 16-byte vectors of a row's columns of one parity
+    const int half = L.s1_pitch >> 1;
+    float* buf = &S.s1[k & 1][0][0][0];
+    for (int i = threadIdx.x; i < kS1TH * 2 * kV; i += kThreads) {
+        const int rr = i / (2 * kV), q = i - rr * (2 * kV);
+        const int par = q >= kV ? 1 : 0, c4 = q - par * kV;
+        const int x = (sx0 >> 1) + 4 * c4, y = sy0 + rr;
+        const bool in = y < L.p1h && x < half;  // x and half are multiples of 4: the whole vector is in the row's half
+        const float* src = in ? base + (long long)y * L.s1_pitch + par * half + x : base;
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + rr * kS1TW + par * (kS1TW / 2) + 4 * c4);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -341,258 +411,288 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// The pooled L2 maps (2i, 2i+1) at tile pixel (x, y), both from S1 map i (the buffer T): 3x3 conv +
-// BN/LReLU at the four positions of the 2x2 window, then their max. A warp reads 32 consecutive
-// column pairs of a row (8-byte loads, no bank conflicts).
-__device__ __forceinline__ f2_t pool_l2_pair(const float (*T)[kS1TW], const Stage1W& W, int i, int x, int y, f2_t nz) {
-    f2_t q[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float2 u = *reinterpret_cast<const float2*>(&T[2 * y + r][2 * x]);
-        const float2 v = *reinterpret_cast<const float2*>(&T[2 * y + r][2 * x + 2]);
-        q[r][0] = f2_dup(u.x);
-        q[r][1] = f2_dup(u.y);
-        q[r][2] = f2_dup(v.x);
-        q[r][3] = f2_dup(v.y);
-    }
-    f2_t cv[4];
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        const int dy = d >> 1, dx = d & 1;
-        f2_t acc = f2_mul(q[dy][dx], f2_ld(W.k2p[i][0]), nz);
-#pragma unroll
-        for (int k = 1; k < 9; ++k) acc = f2_add(acc, f2_mul(q[dy + k / 3][dx + k % 3], f2_ld(W.k2p[i][k]), nz));
-        cv[d] = lrelu_bn2(acc, W.a2p[i], nz);
-    }
-    return f2_max4(cv[0], cv[1], cv[2], cv[3]);
+// Two consecutive duplicated parameters by one 16-byte constant load.
+struct Pair16 {
+    f2_t a, b;
+};
+__device__ __forceinline__ Pair16 ld_pair(const float2* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return Pair16{v.x, v.y};
+}
+__device__ __forceinline__ f2_t lrelu_bn_d(f2_t x, const float2* p, f2_t nz) {
+    const Pair16 u = ld_pair(p), v = ld_pair(p + 2);
+    const f2_t c = f2_add(x, u.a);
+    return f2_add(f2_add(f2_mul(u.b, c, nz), f2_mul(v.a, f2_max0(c), nz)), v.b);
 }
 
-// back: one CTA per 32 x 16 tile of response pixels.
-//   A/B map by map: the four S1 maps of the tile (42 x 72 each) pass through two shared-memory
-//      buffers, map k + 1 copied asynchronously while the pooled L2 maps (2k, 2k+1) are computed from
-//      map k on the 35 x 20 halo tile (one packed pair); the neighbour sums are written as soon as
-//      their three maps are known, the two partial sums a pixel still needs kept in registers. Two
-//      S1 maps in shared memory is what lets four blocks share a SM.
-//   C: every thread finishes two vertically adjacent response pixels, every operation packed over
-//      the pair: the 16 L3 maps (4w x 5h), the 52 hidden neurons and the output neuron.
+// Pooled L2 map m at the tile's pixel pair whose input is q: 3x3 conv + BN/LReLU at the four positions
+// of the 2x2 window, then their max.
+__device__ __forceinline__ f2_t pool_l2(const f2_t (*q)[4], const Stage1Back::L2Map& M, f2_t nz) {
+    f2_t w[10];
+#pragma unroll
+    for (int k = 0; k < 10; k += 2) {
+        const Pair16 u = ld_pair(&M.k[k]);
+        w[k] = u.a;
+        w[k + 1] = u.b;
+    }
+    f2_t acc[4];
+#pragma unroll
+    for (int d = 0; d < 4; ++d) acc[d] = f2_mul(q[d >> 1][d & 1], w[0], nz);
+#pragma unroll
+    for (int k = 1; k < 9; ++k)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) acc[d] = f2_add(acc[d], f2_mul(q[(d >> 1) + k / 3][(d & 1) + k % 3], w[k], nz));
+#pragma unroll
+    for (int d = 0; d < 4; ++d) acc[d] = lrelu_bn_d(acc[d], M.a, nz);
+    return f2_max4(acc[0], acc[1], acc[2], acc[3]);
+}
+
+// back: one CTA per 32 x 16 tile of response pixels, every operation packed over the pixels (x, x + 16)
+// of a row, so that no operand has to be duplicated or paired in registers. kPairs pixel pairs a thread
+// in C (256 / kPairs threads): two halve the constant loads a pixel, which share one queue with the
+// shared-memory loads, and suit launches with many tiles a SM; one gives a tile twice the warps.
+// The four S1 maps of the tile (42 x 72 each) pass through shared memory one after the other; for map k
+//   A: the pooled L2 maps 2k and 2k + 1 on the 35 x 20 halo tile, and the neighbour sums whose three maps
+//      are now known (the two partial sums a pixel still needs stay in registers);
+//   C: the L3 maps (4w x 5h) of those sums, the hidden groups whose four L3 maps are now known and their
+//      part of the output sum, all in registers, while S1 map k + 1 is copied (cp.async).
+// Only one S1 map and three sums are ever held, 21 KB, so that registers alone limit the resident blocks.
 // Back tile t of level L as above; g is its global back-tile index (the gate's tile index).
 // kCoherent: the S1 arena was written earlier in the same launch (read through L2).
-// With the learned gate (cells), a warp (32 x 2 response pixels) without a live pixel writes the skip
-// marker instead of computing, the L2 phase computes only the rows live warps read (warp w reads L2
-// rows 2w .. 2w + 5), and every pixel that is not live is written as the skip marker: only live
-// pixels can become candidates, and their inputs are exactly what runs (the front kernel skips the
-// rest of S1).
-template <bool kCoherent>
-__device__ __forceinline__ void back_tile(const Stage1W& W, const Stage1Dup& D, BackSmem& S, const LevelDesc& L, int t, int g,
-                                          const float* __restrict__ s1, float* __restrict__ resp, int* __restrict__ counts, float thr,
-                                          const uint8_t* __restrict__ back_on, const GateCells& cells) {
+// Warps (32 x 2 kPairs response pixels) and L2 rows that only pixels past the map's last row need are
+// skipped. With the learned gate (cells), a warp without a live pixel writes the skip marker instead of
+// computing, A computes only the rows live warps read (a warp's rows and the four after them), and
+// every pixel that is not live is written as the skip marker: only live pixels can become candidates,
+// and their inputs are exactly what runs (the front kernel skips the rest of S1).
+template <int kPairs, bool kCoherent>
+__device__ __forceinline__ void back_tile(const Stage1Back& D, BackSmem& S, const LevelDesc& L, int t, int g, const float* __restrict__ s1,
+                                          float* __restrict__ resp, int* __restrict__ counts, float thr, const uint8_t* __restrict__ back_on,
+                                          const GateCells& cells) {
+    constexpr int kThreads = kK2TileX * kK2TileY / (2 * kPairs);
+    constexpr int kWarps = kThreads / 32, kWarpRows = kK2TileY / kWarps;
+    constexpr int kP2Passes = (kP2Units + kThreads - 1) / kThreads;
     const int ox0 = (t % L.k2_tiles_x) * kK2TileX;
     const int oy0 = (t / L.k2_tiles_x) * kK2TileY;
     if (back_on && !back_on[g]) {  // gated off: responses below any stage-1 threshold
-        for (int i = threadIdx.x; i < kK2TileX * kK2TileY; i += blockDim.x) {
+        for (int i = threadIdx.x; i < kK2TileX * kK2TileY; i += kThreads) {
             const int gx = ox0 + (i & (kK2TileX - 1)), gy = oy0 + i / kK2TileX;
             if (gx < L.ow && gy < L.oh) resp[L.resp_off + (long long)gy * L.ow + gx] = -1e30f;
         }
         return;
     }
     const int sx0 = 2 * ox0, sy0 = 2 * oy0;
-    const f2_t nz = f2_ld(W.negzero);
+    load_back_map_async<kThreads>(S, s1, L, sx0, sy0, 0);
+    load_back_map_async<kThreads>(S, s1, L, sx0, sy0, 1);
+    const f2_t nz = f2_ld(D.negzero);
     const bool gating = gate_gating(cells);
-    __shared__ int s_live[kK2TileY / 2];  // per warp: any live response pixel
+    const int warp = threadIdx.x >> 5;
+    __shared__ int s_live[kWarps];  // per warp: any live response pixel
     if (gating && (threadIdx.x & 31) == 0) {
-        const int ry = oy0 + 2 * (threadIdx.x >> 5);
-        s_live[threadIdx.x >> 5] = gate_live(cells, L, ox0, ox0 + kK2TileX - 1, ry, ry + 1) ? 1 : 0;
+        const int ry = oy0 + kWarpRows * warp;
+        s_live[warp] = gate_live(cells, L, ox0, ox0 + kK2TileX - 1, ry, ry + kWarpRows - 1) ? 1 : 0;
     }
-
-    load_back_map_async(S, s1, L, sx0, sy0, 0);
-    load_back_map_async(S, s1, L, sx0, sy0, 1);
-    uint32_t live = 0xffu;  // live warps
-    // L2 row y is read by warps ceil((y - 5) / 2) .. y / 2
+    // live warps: those with response rows inside the map (with the gate, with a live pixel in them)
+    const int rows = min(kK2TileY, L.oh - oy0);
+    uint32_t live = (1u << ((rows + kWarpRows - 1) / kWarpRows)) - 1u;
+    const int xe = L.ow - ox0 + 3;  // pooled L2 columns from here on feed no response pixel of the map
+    // L2 row y is read by warps ceil((y - kWarpRows - 3) / kWarpRows) .. y / kWarpRows
     auto need_row = [&](int y) {
-        const int wlo = max(0, (y - 5 + 1) >> 1), whi = min(kK2TileY / 2 - 1, y >> 1);
-        return wlo <= whi && ((live >> wlo) & ((1u << (whi - wlo + 1)) - 1u)) != 0u;
+        const int wlo = max(0, y - (kWarpRows + 3) + kWarpRows - 1) / kWarpRows, whi = min(kWarps - 1, y / kWarpRows);
+        return ((live >> wlo) & ((1u << (whi - wlo + 1)) - 1u)) != 0u;
     };
-    // pooled L2 maps (2k, 2k+1) = (A, B) from S1 map k; the sums in the reference's order:
-    // s0 = P0 + P1, s1 = s0 + P2, s(2j) = (P(2j-1) + P(2j)) + P(2j+1), s(2j+1) = (P(2j) + P(2j+1)) + P(2j+2),
-    // s7 = P6 + P7; ca and cb carry (P(2k) + P(2k+1)) and P(2k+1) to the next map
-    float ca[kP2Passes], cb[kP2Passes];
-#pragma unroll
+    // the thread's response pixels: (x, x + 16) of rows y .. y + kPairs - 1
+    const int x = threadIdx.x & (kHalfX - 1), y = (threadIdx.x / kHalfX) * kPairs;
+    const f2_t half = f2_pack(0.5f, 0.5f);
+    // A: the sums in the reference's order: s0 = P0 + P1, s1 = s0 + P2, s(2j) = (P(2j-1) + P(2j)) + P(2j+1),
+    // s(2j+1) = (P(2j) + P(2j+1)) + P(2j+2), s7 = P6 + P7; ca and cb carry (P(2k) + P(2k+1)) and P(2k+1)
+    // to the next map
+    f2_t ca[kP2Passes], cb[kP2Passes];
+    // C: hidden neuron n = 4*i + t reads L3 maps i..i+3: a[0]..a[3] is the window of the last four L3 maps;
+    // the output sum runs over n in order
+    static_assert(Stage1W::kConn == 4 && Stage1W::kGroups + 3 == Stage1W::kM3, "sliding window of four L3 maps");
+    f2_t a[4][kPairs] = {}, out[kPairs] = {};
+#pragma unroll 1
     for (int k = 0; k < 4; ++k) {
-        if (k == 0)
-            cp_async_wait<1>();
-        else
-            cp_async_wait<0>();
-        __syncthreads();  // map k is in shared memory for every thread, and map k - 1's buffer is free
+        if (k < 3) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        __syncthreads();  // S1 map k is in shared memory for every thread, and the sums of map k - 1 are read
         if (k == 0 && gating) {
-            live = 0u;
+            uint32_t on = 0u;
 #pragma unroll
-            for (int w = 0; w < kK2TileY / 2; ++w) live |= (s_live[w] ? 1u : 0u) << w;
+            for (int w = 0; w < kWarps; ++w) on |= (s_live[w] ? 1u : 0u) << w;
+            live &= on;
         }
-        if (k == 1 || k == 2) load_back_map_async(S, s1, L, sx0, sy0, k + 1);
-        const float(*T)[kS1TW] = S.s1[k & 1];
+        const float(*T)[2][kS1TW / 2] = S.s1[k & 1];
 #pragma unroll
         for (int kk = 0; kk < kP2Passes; ++kk) {
-            const int p = threadIdx.x + 256 * kk;
-            int x = 0, y = 0;
-            if (p < kP2Px) p2_pixel(p, &x, &y);
-            if (p < kP2Px && need_row(y)) {
-                const f2_t a = pool_l2_pair(T, W, k, x, y, nz);
-                const float A = f2_lo(a), B = f2_hi(a);
+            const int p = threadIdx.x + kThreads * kk;
+            int ux = 0, uy = 0;
+            if (p < kP2Units) p2_unit(p, &ux, &uy);
+            if (p < kP2Units && ux < xe && need_row(uy)) {
+                f2_t q[4][4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        q[r][c] = f2_pack(T[2 * uy + r][c & 1][ux + (c >> 1)], T[2 * uy + r][c & 1][ux + kHalfX + (c >> 1)]);
+                const f2_t A = pool_l2(q, D.l2[2 * k], nz), B = pool_l2(q, D.l2[2 * k + 1], nz);
+                auto put = [&](int slot, f2_t v) { *reinterpret_cast<f2_t*>(&S.s2[slot][uy][ux]) = v; };
+                const f2_t ab = f2_add(A, B);
                 if (k == 0) {
-                    const float s01 = fadd(A, B);
-                    S.s2[0][y][x] = s01;
-                    ca[kk] = s01;
+                    put(0, ab);
                 } else {
-                    S.s2[2 * k - 1][y][x] = fadd(ca[kk], A);
-                    S.s2[2 * k][y][x] = fadd(fadd(cb[kk], A), B);
-                    if (k < 3) ca[kk] = fadd(A, B);
-                    else S.s2[7][y][x] = fadd(A, B);
+                    put(0, f2_add(ca[kk], A));
+                    put(1, f2_add(f2_add(cb[kk], A), B));
+                    if (k == 3) put(2, ab);
                 }
+                ca[kk] = ab;
                 cb[kk] = B;
             }
         }
-    }
-    __syncthreads();
-
-    // C: pixels (x, y) and (x, y + 1)
-    const int x = threadIdx.x & (kK2TileX - 1), y = (threadIdx.x / kK2TileX) * 2;
-    if (!((live >> (threadIdx.x >> 5)) & 1u)) {
-        // no live pixel in the warp: the skip marker instead of the responses
-        const int gx = ox0 + x, gy = oy0 + y;
-        if (gx < L.ow) {
-            if (gy < L.oh) resp[L.resp_off + (long long)gy * L.ow + gx] = -1e30f;
-            if (gy + 1 < L.oh) resp[L.resp_off + (long long)(gy + 1) * L.ow + gx] = -1e30f;
-        }
-        return;
-    }
-    // L3 maps (2k, 2k+1) of the pixel pair, both from neighbour-sum map k; conv_5x4 keeps one
-    // partial sum per kernel row, added in row order
-    auto l3_pair = [&](int k, f2_t* m0, f2_t* m1) {
-        float v[6][4];
-#pragma unroll
-        for (int r = 0; r < 6; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) v[r][c] = S.s2[k][y + r][x + c];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int mm = 2 * k + e;
-            f2_t acc = 0ull;
-#pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                f2_t rs = f2_mul(f2_pack(v[r][0], v[r + 1][0]), f2_ld(D.k3d[mm][4 * r]), nz);
-#pragma unroll
-                for (int c = 1; c < 4; ++c) rs = f2_add(rs, f2_mul(f2_pack(v[r][c], v[r + 1][c]), f2_ld(D.k3d[mm][4 * r + c]), nz));
-                acc = (r == 0) ? rs : f2_add(acc, rs);
-            }
-            *(e == 0 ? m0 : m1) = lrelu_bn2(acc, D.a3d[mm], nz);
-        }
-    };
-    // hidden neuron n = 4*i + t reads L3 maps i..i+3: the groups run as a loop over a sliding window
-    // of four maps (a0..a3, with the second map of the last computed pair kept in `spare`), so the
-    // code stays small; the output sum runs over n in order
-    static_assert(Stage1W::kConn == 4 && Stage1W::kGroups + 3 == Stage1W::kM3, "sliding window of four L3 maps");
-    f2_t a0, a1, a2, a3, spare;
-    l3_pair(0, &a0, &a1);
-    l3_pair(1, &a2, &spare);
-    const f2_t half = f2_pack(0.5f, 0.5f);
-    f2_t out = 0ull;
+        __syncthreads();  // the sums are complete, and map k's buffer is free
+        if (k < 2) load_back_map_async<kThreads>(S, s1, L, sx0, sy0, k + 2);
+        if (!((live >> warp) & 1u)) continue;
+        const int first = k == 0 ? 0 : 2 * k - 1, n_sums = k == 0 ? 1 : (k == 3 ? 3 : 2);
 #pragma unroll 1
-    for (int i = 0; i < Stage1W::kGroups; ++i) {
-        const int m = i + 3;  // the group's newest map
-        if (m & 1) a3 = spare;
-        else l3_pair(m >> 1, &a3, &spare);
+        for (int j = 0; j < n_sums; ++j) {
+            // L3 maps (2s, 2s+1) of the pixel pairs from sum s; conv_5x4 keeps one partial sum per kernel
+            // row, added in row order
+            const int s = first + j;
+            f2_t nm[2][kPairs];
+            {
+                f2_t acc[2][kPairs], v[kPairs][4];
 #pragma unroll
-        for (int tt = 0; tt < Stage1W::kHS; ++tt) {
-            const int n = Stage1W::kHS * i + tt;
-            f2_t s = f2_ld(D.hbd[n]);
-            s = f2_add(s, f2_mul(a0, f2_ld(D.hwd[n][0]), nz));
-            s = f2_add(s, f2_mul(a1, f2_ld(D.hwd[n][1]), nz));
-            s = f2_add(s, f2_mul(a2, f2_ld(D.hwd[n][2]), nz));
-            s = f2_add(s, f2_mul(a3, f2_ld(D.hwd[n][3]), nz));
-            s = f2_mul(s, f2_ld(D.htwd[i]), nz);
-            f2_t v = tanh_rational2(s, nz);
-            v = f2_add(f2_mul(half, v, nz), half);
-            const f2_t h = f2_add(f2_mul(f2_ld(D.hbnwd[tt]), v, nz), f2_ld(D.hbnbd[tt]));
-            const f2_t hw = f2_mul(h, f2_ld(D.owd[n]), nz);
-            out = (n == 0) ? hw : f2_add(hw, out);
+                for (int p = 0; p < kPairs - 1; ++p)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[p][c] = f2_ld(S.s2[j][y + p][x + c]);
+#pragma unroll
+                for (int r = 0; r < 5; ++r) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[kPairs - 1][c] = f2_ld(S.s2[j][y + r + kPairs - 1][x + c]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const Pair16 w01 = ld_pair(&D.l3[2 * s + e].k[4 * r]), w23 = ld_pair(&D.l3[2 * s + e].k[4 * r + 2]);
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) {
+                            f2_t rs = f2_mul(v[p][0], w01.a, nz);
+                            rs = f2_add(rs, f2_mul(v[p][1], w01.b, nz));
+                            rs = f2_add(rs, f2_mul(v[p][2], w23.a, nz));
+                            rs = f2_add(rs, f2_mul(v[p][3], w23.b, nz));
+                            acc[e][p] = (r == 0) ? rs : f2_add(acc[e][p], rs);
+                        }
+                    }
+#pragma unroll
+                    for (int p = 0; p < kPairs - 1; ++p)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) v[p][c] = v[p + 1][c];
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int p = 0; p < kPairs; ++p) nm[e][p] = lrelu_bn_d(acc[e][p], D.l3[2 * s + e].a, nz);
+            }
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                for (int p = 0; p < kPairs; ++p) {
+                    a[0][p] = a[1][p];
+                    a[1][p] = a[2][p];
+                    a[2][p] = a[3][p];
+                    a[3][p] = nm[0][p];
+                    nm[0][p] = nm[1][p];
+                }
+                const int i = 2 * s + e - 3;  // the hidden group that L3 map 2s + e completes
+                if (i < 0) continue;
+                const f2_t tw = f2_ld(D.htw[i]);
+#pragma unroll
+                for (int tt = 0; tt < Stage1W::kHS; ++tt) {
+                    const int n = Stage1W::kHS * i + tt;
+                    const Stage1Back::Neuron& N = D.hid[n];
+                    const Pair16 bw = ld_pair(&N.b), w12 = ld_pair(&N.w[1]), w3o = ld_pair(&N.w[3]), bn = ld_pair(&D.hbn[tt].w);
+#pragma unroll
+                    for (int p = 0; p < kPairs; ++p) {
+                        f2_t h = f2_add(bw.a, f2_mul(a[0][p], bw.b, nz));
+                        h = f2_add(h, f2_mul(a[1][p], w12.a, nz));
+                        h = f2_add(h, f2_mul(a[2][p], w12.b, nz));
+                        h = f2_add(h, f2_mul(a[3][p], w3o.a, nz));
+                        const f2_t v = tanh_half2(f2_mul(h, tw, nz), nz, half);
+                        const f2_t hw = f2_mul(f2_add(f2_mul(bn.a, v, nz), bn.b), w3o.b, nz);
+                        out[p] = (n == 0) ? hw : f2_add(hw, out[p]);
+                    }
+                }
+            }
         }
-        a0 = a1;
-        a1 = a2;
-        a2 = a3;
     }
-    f2_t c = f2_mul(f2_add(out, f2_ld(D.obd)), f2_ld(D.otwd), nz);
-    c = tanh_rational2(c, nz);
-    const f2_t r = (W.af == 0.f) ? f2_add(f2_mul(half, c, nz), half) : f2_mul(f2_ld(D.afd), c, nz);
     const int gx = ox0 + x, gy = oy0 + y;
-    if (gx < L.ow) {
-        float rv[2] = {f2_lo(r), f2_hi(r)};
-        if (gating) {
+    const bool on = (live >> warp) & 1u;  // else the skip marker instead of the responses
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        f2_t c = f2_mul(f2_add(out[p], f2_ld(D.ob)), f2_ld(D.otw), nz);
+        c = tanh_rational2(c, nz);
+        const f2_t r = D.half_out ? f2_add(f2_mul(half, c, nz), half) : f2_mul(f2_ld(D.af), c, nz);
+        if (gy + p >= L.oh) break;
+        const int at = (gy + p) * L.ow + gx;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int px = gx + h * kHalfX;
+            if (px >= L.ow) break;
+            float v = h == 0 ? f2_lo(r) : f2_hi(r);
             // only live pixels keep their response (a candidate needs a likely cell of its octave within
             // the margin of its window centre); the others may have read skipped inputs
-            for (int k = 0; k < 2; ++k)
-                if (!gate_live(cells, L, gx, gx, gy + k, gy + k)) rv[k] = -1e30f;
-        }
-        // candidates (response > treshold_1) are counted per scan chunk for the compaction
-        if (gy < L.oh) {
-            resp[L.resp_off + (long long)gy * L.ow + gx] = rv[0];
-            if (counts && rv[0] > thr) atomicAdd(&counts[L.chunk_base + (gy * L.ow + gx) / kCandChunk], 1);
-        }
-        if (gy + 1 < L.oh) {
-            resp[L.resp_off + (long long)(gy + 1) * L.ow + gx] = rv[1];
-            if (counts && rv[1] > thr) atomicAdd(&counts[L.chunk_base + ((gy + 1) * L.ow + gx) / kCandChunk], 1);
+            if (!on || (gating && !gate_live(cells, L, px, px, gy + p, gy + p))) v = -1e30f;
+            resp[L.resp_off + at + h * kHalfX] = v;
+            // candidates (response > treshold_1) are counted per scan chunk for the compaction
+            if (counts && v > thr) atomicAdd(&counts[L.chunk_base + (at + h * kHalfX) / kCandChunk], 1);
         }
     }
 }
 
-template <int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) stage1_back_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ Stage1Dup D,
-                                                             const __grid_constant__ LevelTable LT, const float* __restrict__ s1,
-                                                             float* __restrict__ resp, int* __restrict__ counts, float thr,
-                                                             const uint8_t* __restrict__ back_on, const GateCells cells) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BackSmem& S = *reinterpret_cast<BackSmem*>(smem_raw);
+template <int kPairs, int kMinBlocks>
+__global__ void __launch_bounds__(256 / kPairs, kMinBlocks) stage1_back_kernel(const __grid_constant__ Stage1Back D, const __grid_constant__ LevelTable LT,
+                                                             const float* __restrict__ s1, float* __restrict__ resp, int* __restrict__ counts,
+                                                             float thr, const uint8_t* __restrict__ back_on, const GateCells cells) {
+    __shared__ BackSmem S;
     const int g = LT.first + blockIdx.x;
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k2_base>(LT, g)];
     const int t = g - L.k2_base;
-    back_tile<false>(W, D, S, L, t, g, s1, resp, counts, thr, back_on, cells);
+    back_tile<kPairs, false>(D, S, L, t, g, s1, resp, counts, thr, back_on, cells);
 }
 
-// Duplicated stage-1 parameters for the back kernel, derived from the packed weight block.
-static Stage1Dup make_dup(const Stage1W& W) {
-    Stage1Dup D;
+// The back kernel's parameters, derived from the packed weight block.
+static Stage1Back make_back(const Stage1W& W) {
+    Stage1Back D{};
     auto dup = [](float v) { return make_float2(v, v); };
-    for (int i = 0; i < Stage1W::kM3 / 2; ++i)
-        for (int k = 0; k < Stage1W::kK3W * Stage1W::kK3H; ++k) {
-            D.k3d[2 * i][k] = dup(W.k3p[i][k].x);
-            D.k3d[2 * i + 1][k] = dup(W.k3p[i][k].y);
-        }
-    for (int mm = 0; mm < Stage1W::kM3; ++mm) {
-        D.a3d[mm][0] = dup(W.b3[mm]);
-        D.a3d[mm][1] = dup(W.w3a[mm]);
-        D.a3d[mm][2] = dup(W.w3b[mm]);
-        D.a3d[mm][3] = dup(W.bn3[mm]);
+    auto act = [&](float2* a, float b, float wa, float wb, float bn) {
+        a[0] = dup(b);
+        a[1] = dup(wa);
+        a[2] = dup(wb);
+        a[3] = dup(bn);
+    };
+    for (int m = 0; m < Stage1W::kM2; ++m) {
+        for (int k = 0; k < Stage1W::kK2W * Stage1W::kK2H; ++k) D.l2[m].k[k] = dup((m & 1) ? W.k2p[m / 2][k].y : W.k2p[m / 2][k].x);
+        act(D.l2[m].a, W.b2[m], W.w2a[m], W.w2b[m], W.bn2[m]);
     }
-    for (int q = 0; q < Stage1W::kHL / 2; ++q)
-        for (int j = 0; j < Stage1W::kConn; ++j) {
-            D.hwd[2 * q][j] = dup(W.hwp[q][j].x);
-            D.hwd[2 * q + 1][j] = dup(W.hwp[q][j].y);
-        }
+    for (int m = 0; m < Stage1W::kM3; ++m) {
+        for (int k = 0; k < Stage1W::kK3W * Stage1W::kK3H; ++k) D.l3[m].k[k] = dup((m & 1) ? W.k3p[m / 2][k].y : W.k3p[m / 2][k].x);
+        act(D.l3[m].a, W.b3[m], W.w3a[m], W.w3b[m], W.bn3[m]);
+    }
     for (int n = 0; n < Stage1W::kHL; ++n) {
-        D.hbd[n] = dup(W.hb[n]);
-        D.owd[n] = dup(W.ow[n]);
+        D.hid[n].b = dup(W.hb[n]);
+        for (int j = 0; j < Stage1W::kConn; ++j) D.hid[n].w[j] = dup((n & 1) ? W.hwp[n / 2][j].y : W.hwp[n / 2][j].x);
+        D.hid[n].o = dup(W.ow[n]);
     }
-    for (int i = 0; i < Stage1W::kGroups; ++i) D.htwd[i] = dup(W.htw[i]);
-    for (int tt = 0; tt < Stage1W::kHS; ++tt) {
-        D.hbnwd[tt] = dup(W.hbnw[tt]);
-        D.hbnbd[tt] = dup(W.hbnb[tt]);
+    for (int i = 0; i < Stage1W::kGroups; ++i) D.htw[i] = dup(W.htw[i]);
+    for (int t = 0; t < Stage1W::kHS; ++t) {
+        D.hbn[t].w = dup(W.hbnw[t]);
+        D.hbn[t].b = dup(W.hbnb[t]);
     }
-    D.obd = dup(W.ob);
-    D.otwd = dup(W.otw);
-    D.afd = dup(W.af);
+    D.ob = dup(W.ob);
+    D.otw = dup(W.otw);
+    D.af = dup(W.af);
+    D.negzero = W.negzero;
+    D.half_out = W.af == 0.f ? 1 : 0;
     return D;
 }
-
-
 
 // Launches KERNEL once per group of at most kParamLevels levels; tiles(L) is a level's block count
 // and base(L) its first global block.
@@ -617,26 +717,36 @@ cudaError_t launch_stage1_front(const Stage1W& W, const LevelDesc* levels, int n
     return launch_grouped(
         levels, n_levels, &LevelDesc::k1_base, [](const LevelDesc& L) { return L.k1_tiles_x * ((L.p1h + kK1TileY - 1) / kK1TileY); },
         [&](const LevelTable& T, int blocks) {
-            const bool four = sched.front_blocks_per_sm >= 4;
+            const bool six = sched.front_blocks_per_sm >= 4;
             if (gray.p)
-                (four ? stage1_front_kernel<true, 4> : stage1_front_kernel<true, 3>)<<<blocks, 256, 0, st>>>(W, T, limg, gray, s1, front_on,
-                                                                                                              cells);
+                (six ? stage1_front_kernel<true, 6> : stage1_front_kernel<true, 5>)<<<blocks, kFrontThreads, 0, st>>>(W, T, limg, gray, s1, front_on, cells);
             else
-                (four ? stage1_front_kernel<false, 4> : stage1_front_kernel<false, 3>)<<<blocks, 256, 0, st>>>(W, T, limg, gray, s1, front_on,
-                                                                                                                cells);
+                (six ? stage1_front_kernel<false, 6> : stage1_front_kernel<false, 5>)<<<blocks, kFrontThreads, 0, st>>>(W, T, limg, gray, s1, front_on,
+                                                                                                                         cells);
         });
 }
 
 cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* s1, float* resp, cudaStream_t st,
                                int* counts, float thr, const uint8_t* back_on, GateCells cells, Stage1Sched sched) {
-    const Stage1Dup D = make_dup(W);
+    const Stage1Back D = make_back(W);
+    if (n_levels <= 0) return cudaSuccess;
+    // Two pixel pairs a thread do the same work with 8 % fewer instructions, but a tile then has 4 warps
+    // instead of 8 and takes longer by itself. They are used where every SM has at least two tiles to run
+    // (3840x2160, scale 1.05: 1.34 ms a frame against 1.72; 1080p: 53 us against 61); below that, and
+    // with the learned gate, which runs about a quarter of the tiles and skips by warps of 32 x 2 pixels
+    // instead of 32 x 4, one pair (640x480: 27.6 us against 29.6; a gated 1080p frame 37 us against 43).
+    constexpr int kTwoPairTiles = 296;
+    const LevelDesc& last = levels[n_levels - 1];
+    const int tiles = last.k2_base + last.k2_tiles_x * ((last.oh + kK2TileY - 1) / kK2TileY);
+    const bool two_pairs = tiles >= kTwoPairTiles && !back_on;
     return launch_grouped(
         levels, n_levels, &LevelDesc::k2_base, [](const LevelDesc& L) { return L.k2_tiles_x * ((L.oh + kK2TileY - 1) / kK2TileY); },
         [&](const LevelTable& T, int blocks) {
-            if (sched.back_blocks_per_sm >= 4)
-                stage1_back_kernel<4><<<blocks, 256, kBackSmemBytes, st>>>(W, D, T, s1, resp, counts, thr, back_on, cells);
+            if (two_pairs)
+                (sched.back_blocks_per_sm >= 4 ? stage1_back_kernel<2, 6> : stage1_back_kernel<2, 5>)<<<blocks, 128, 0, st>>>(D, T, s1, resp, counts, thr,
+                                                                                                                               back_on, cells);
             else
-                stage1_back_kernel<3><<<blocks, 256, kBackSmemBytes, st>>>(W, D, T, s1, resp, counts, thr, back_on, cells);
+                stage1_back_kernel<1, 3><<<blocks, 256, 0, st>>>(D, T, s1, resp, counts, thr, back_on, cells);
         });
 }
 
@@ -692,10 +802,10 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
     return v;
 }
 
+constexpr int kBatchThreads = kFrontThreads;  // a front tile's block, and a back tile's with two pairs a thread
 constexpr int kBatchSmem = (int)sizeof(BackSmem) > (int)sizeof(FrontSmem) ? (int)sizeof(BackSmem) : (int)sizeof(FrontSmem);
 
-template <int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) stage1_batch_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ Stage1Dup D,
+__global__ void __launch_bounds__(kBatchThreads, 5) stage1_batch_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ Stage1Back D,
                                                               const __grid_constant__ BatchFrames F, const __grid_constant__ BatchQueue Q,
                                                               const LevelDesc* __restrict__ levels, int* __restrict__ sync,
                                                               int* __restrict__ err) {
@@ -748,10 +858,10 @@ __global__ void __launch_bounds__(256, kMinBlocks) stage1_batch_kernel(const __g
         const LevelDesc& L = levels[lo];
         if (stage == 0) {
             if (!F.front_on[f] || F.front_on[f][g])
-                front_tile<true, false>(W, *reinterpret_cast<FrontSmem*>(smem_raw), L, g - L.k1_base, nullptr,
+                front_tile<true>(W, *reinterpret_cast<FrontSmem*>(smem_raw), L, g - L.k1_base, nullptr,
                                         GrayRef{F.gray[f], F.gpitch, F.gw, F.gh}, F.s1[f], F.cells[f]);
         } else {
-            back_tile<true>(W, D, *reinterpret_cast<BackSmem*>(smem_raw), L, g - L.k2_base, g, F.s1[f], F.resp[f], F.counts[f], Q.thr,
+            back_tile<2, true>(D, *reinterpret_cast<BackSmem*>(smem_raw), L, g - L.k2_base, g, F.s1[f], F.resp[f], F.counts[f], Q.thr,
                             F.back_on[f], F.cells[f]);
         }
         __syncthreads();  // every thread is done with the item (and with the shared memory)
@@ -778,35 +888,31 @@ cudaError_t launch_counts_zero_batch(const BatchFrames& F, int n_chunks, int n_f
     return cudaGetLastError();
 }
 
-// resident blocks per SM of the persistent kernel: the schedule's count (1-4), at most what fits
+// resident blocks per SM of the persistent kernel: twice the schedule's count (1-4, in units of 256
+// threads), at most what fits
 int stage1_batch_blocks_per_sm(int blocks_per_sm) {
     int n = 0;
-    if (blocks_per_sm >= 4)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage1_batch_kernel<4>, 256, kBatchSmem);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage1_batch_kernel<3>, 256, kBatchSmem);
-    if (blocks_per_sm >= 1 && blocks_per_sm < n) n = blocks_per_sm;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage1_batch_kernel, kBatchThreads, kBatchSmem);
+    if (blocks_per_sm >= 1 && 2 * blocks_per_sm < n) n = 2 * blocks_per_sm;
     return n > 0 ? n : 1;
 }
 
 cudaError_t launch_stage1_batch(const Stage1W& W, const BatchFrames& F, const BatchQueue& Q, const LevelDesc* d_levels, int* sync, int* err,
-                                int grid, cudaStream_t st, int blocks_per_sm) {
+                                int grid, cudaStream_t st) {
     if (Q.total <= 0) return cudaSuccess;
     if (Q.n_levels > kMaxBatchLevels) return cudaErrorInvalidValue;
-    const Stage1Dup D = make_dup(W);
+    const Stage1Back D = make_back(W);
     grid = grid < Q.total ? grid : Q.total;
-    if (blocks_per_sm >= 4)
-        stage1_batch_kernel<4><<<grid, 256, kBatchSmem, st>>>(W, D, F, Q, d_levels, sync, err);
-    else
-        stage1_batch_kernel<3><<<grid, 256, kBatchSmem, st>>>(W, D, F, Q, d_levels, sync, err);
+    stage1_batch_kernel<<<grid, kBatchThreads, kBatchSmem, st>>>(W, D, F, Q, d_levels, sync, err);
     return cudaGetLastError();
 }
 
+// The back kernels' resident blocks need most of a SM's 228 KB as shared memory (33 KB each).
 cudaError_t stage1_setup() {
-    cudaError_t e = cudaFuncSetAttribute(stage1_back_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage1_back_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage1_batch_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage1_batch_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
+    const auto prefer = [](const void* f) { return cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); };
+    cudaError_t e = prefer(reinterpret_cast<const void*>(stage1_back_kernel<1, 3>));
+    if (e == cudaSuccess) e = prefer(reinterpret_cast<const void*>(stage1_back_kernel<2, 5>));
+    if (e == cudaSuccess) e = prefer(reinterpret_cast<const void*>(stage1_back_kernel<2, 6>));
     return e;
 }
 

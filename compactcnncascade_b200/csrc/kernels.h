@@ -126,7 +126,7 @@ void build_batch_queue(BatchQueue* q, int n_frames, int n_levels, int n_chunks, 
 // Front items resample their level tiles from the gray frames (the pyramid is never stored); the
 // candidate counts must be zero (launch_counts_zero_batch).
 cudaError_t launch_stage1_batch(const Stage1W& W, const BatchFrames& F, const BatchQueue& Q, const LevelDesc* d_levels, int* sync, int* err,
-                                int grid, cudaStream_t st, int blocks_per_sm);
+                                int grid, cudaStream_t st);
 // levels of a pyramid the persistent stage-1 kernel takes (their first items live in shared memory);
 // deeper pyramids run the per-level kernels
 constexpr int kMaxBatchLevels = 256;
@@ -161,7 +161,9 @@ cudaError_t launch_window_batch(const WindowNets& N, const WinBatch& B, int gpit
 // the replay of every frame of a batch: block f runs args[f] (device memory)
 cudaError_t launch_replay_batch(const ReplayArgs* d_args, int n_frames, cudaStream_t st);
 
-// register budget of the stage-1 kernels: resident 256-thread blocks per SM (3 or 4), a schedule knob
+// register budget of the stage-1 kernels, a schedule knob: 3 or 4, in units of 256 threads a SM at about 80
+// and 64 registers (the kernels' own blocks: front 5 or 6 of 128 threads, back 5 or 6 of 128 threads where it
+// runs two pixel pairs a thread)
 struct Stage1Sched {
     int front_blocks_per_sm = 3;
     int back_blocks_per_sm = 4;
@@ -186,7 +188,7 @@ cudaError_t launch_stage1(const Stage1W& W, const LevelDesc* levels, int n_level
 cudaError_t launch_stage1_front(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* limg, float* s1, cudaStream_t st,
                                 const uint8_t* front_on = nullptr, Stage1Sched sched = Stage1Sched{}, GrayRef gray = GrayRef{},
                                 GateCells cells = GateCells{});
-// dynamic shared memory of the stage-1 back kernel (set once per device before any launch)
+// shared-memory carve-out of the stage-1 back kernels (once per device before any launch)
 cudaError_t stage1_setup();
 cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* s1, float* resp, cudaStream_t st,
                                int* counts = nullptr, float thr = 0.f, const uint8_t* back_on = nullptr, GateCells cells = GateCells{},
