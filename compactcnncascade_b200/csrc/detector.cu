@@ -493,11 +493,11 @@ ccnn_status Detector::build_plan(int w, int h, int ch, int num_scales, Plan* p) 
         L.s1_off = s1;
         s1 += 4 * L.s1_plane;
         if (legacy_) {
-            // the legacy stage-1 network's response map, and its pooled L1 and L2 maps in the S1 arena
+            // the legacy stage-1 network's response map, and its sums of pooled L2 maps in the S1 arena
             const LegacyNet& n = h_lg_[0];
             legacy_output_size(n, L.w, L.h, &L.ow, &L.oh);
             s1 -= 4 * L.s1_plane;  // L.s1_off stays this level's start
-            s1 += (long long)n.m0 * L.p1w * L.p1h + (long long)n.m1 * L.p2w * L.p2h;
+            s1 += (long long)legacy_scratch_floats(n, L.w, L.h);
         }
         L.resp_off = resp;
         resp += (long long)L.ow * L.oh;
@@ -834,14 +834,15 @@ ccnn_status Detector::enqueue_kernels(Slot& s, const Plan& p) {
     return CCNN_OK;
 }
 
-// Stage 1 of the legacy family: the legacy network on every level image, its pooled maps in the
+// Stage 1 of the legacy family: the legacy network on every level image, its sums of pooled maps in the
 // S1 arena, candidates counted per scan chunk.
 ccnn_status Detector::enqueue_legacy_stage1(Slot& s, const Plan& p) {
+    std::vector<LegacyLevel> lv(p.n_levels);
     for (int i = 0; i < p.n_levels; ++i) {
         const LevelDesc& L = p.levels[i];
-        CCNN_CUDA(launch_legacy_forward(d_lg_, h_lg_[0], s.d_limg + L.img_off, L.img_pitch, L.w, L.h, s.d_s1 + L.s1_off, s.d_resp + L.resp_off, s.st,
-                                        s.d_counts, L.chunk_base, cfg_.thr1));
+        lv[i] = LegacyLevel{s.d_limg + L.img_off, L.img_pitch, L.w, L.h, s.d_s1 + L.s1_off, s.d_resp + L.resp_off, L.chunk_base};
     }
+    CCNN_CUDA(launch_legacy_forward(d_lg_, h_lg_[0], lv.data(), p.n_levels, s.st, s.d_counts, cfg_.thr1));
     return CCNN_OK;
 }
 

@@ -11,8 +11,8 @@
 //     mulC2_add / mulC1_add / tanh :968-1002, :868) summed over the neurons,
 //   and the output tanh(sum + bias) * af (tanh :868).
 // tanh is the reference's rational form sgn(c) (1 - 1 / (1 + |c| + c^2 + 1.41645 c^4)) (USE_FAST_TANH).
-// One thread computes one pooled pixel of one map (L1, L2) or one response pixel (L3 onwards);
-// neighbouring-map sums are recomputed where they are read, with the reference's additions.
+// Two kernels over all levels: L1 and L2 with the neighbouring-map sums, and L3 to the output. Maps
+// (2i, 2i + 1) read the same input and run as packed pairs, each lane with the reference's roundings.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -22,8 +22,7 @@
 #include <vector>
 
 #include "../../include/ccnn_inspect.h"
-#include "ccnn_common.cuh"
-#include "legacy.h"
+#include "kernels.h"
 #include "legacy_dev.cuh"
 
 namespace ccnn {
@@ -146,99 +145,248 @@ bool load_legacy_model_file(const std::string& path, LegacyNet* net, std::string
 
 namespace {
 
-__global__ void legacy_l1_kernel(const LegacyNet* __restrict__ N, const float* __restrict__ img, int pitch, int p1w, int p1h,
-                                 float* __restrict__ pool1) {
-    const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y, m = blockIdx.z;
-    if (px >= p1w || py >= p1h) return;
-    const float* k = N->k1[m];
-    float c[4];
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        const float* s = img + (size_t)(2 * py + (d >> 1)) * pitch + 2 * px + (d & 1);
-        float acc = fmul(s[0], k[0]);
-#pragma unroll
-        for (int t = 1; t < 16; ++t) acc = fadd(acc, fmul(s[(t >> 2) * pitch + (t & 3)], k[t]));
-        c[d] = acc;
-    }
-    pool1[((long long)m * p1h + py) * p1w + px] = lg_pool_tanh(c, N->max_pool, N->cb[0][m], N->sw[0][m], N->sb[0][m], N->af);
+constexpr int kLgT = 256;              // threads
+constexpr int kLgTX = 32, kLgTY = 8;   // pooled L2 pixels, or responses, of a block
+constexpr int kLgLevels = 32;          // levels a launch (its table travels as a kernel parameter)
+constexpr int kLgP1X = 2 * kLgTX + 2, kLgP1Y = 2 * kLgTY + 2;  // pooled L1 pixels that a tile of L2 reads
+constexpr int kLgP1S = kLgP1X + 1;                             // row stride of their sums
+
+// The levels of one launch and each one's first block: `pool` for the L1 and L2 layers, `out` for the rest.
+struct LgTable {
+    int n;
+    struct Level {
+        LegacyLevel L;
+        int p2w, p2h, ow, oh;
+        int pool_base, pool_tx, out_base, out_tx;
+    } lv[kLgLevels];
+};
+
+template <int LgTable::Level::* base>
+__device__ __forceinline__ const LgTable::Level& lg_level(const LgTable& T, int block) {
+    int i = 0;
+    while (i + 1 < T.n && block >= T.lv[i + 1].*base) ++i;
+    return T.lv[i];
 }
 
-__global__ void legacy_l2_kernel(const LegacyNet* __restrict__ N, const float* __restrict__ pool1, int p1w, int p1h, int p2w, int p2h,
-                                 float* __restrict__ pool2) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y, m = blockIdx.z;
-    if (x >= p2w || y >= p2h) return;
-    const int i = m >> 1;
-    const long long plane = (long long)p1w * p1h;
-    float S[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) S[r][q] = lg_map_sum(pool1, plane, N->m0, i, (long long)(2 * y + r) * p1w + 2 * x + q);
-    const float* k = N->k2[m];
-    float c[4];
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        const int dy = d >> 1, dx = d & 1;
-        float acc = fmul(S[dy][dx], k[0]);
-#pragma unroll
-        for (int t = 1; t < 9; ++t) acc = fadd(acc, fmul(S[dy + t / 3][dx + t % 3], k[t]));
-        c[d] = acc;
+// L1, the sums of neighbouring L1 maps, L2 and the sums of neighbouring L2 maps (which L3 reads) of one
+// 32 x 8 tile of pooled L2 pixels; the L1 sums stay in shared memory. A thread computes every map of its
+// pixel, two at a time (packed; an odd last map's partner is computed with zero weights and dropped). Bound by
+// latency: a 640 x 480 frame's levels are about one block a SM.
+__global__ void __launch_bounds__(kLgT) legacy_pool_kernel(const LegacyNet* __restrict__ N, const __grid_constant__ LgTable T, const f2_t nz) {
+    __shared__ float s1[kLgMaxM0][kLgP1Y][kLgP1S];
+    __shared__ float2 k1[kLgMaxM0 / 2][16], k2[kLgMaxM0][9];
+    __shared__ LgPoolPair q1[kLgMaxM0 / 2], q2[kLgMaxM0];
+    const int tid = threadIdx.x;
+    const int m0 = N->m0, max_pool = N->max_pool;
+    for (int i = tid; i < kLgMaxM0 / 2 * 16; i += kLgT) {
+        const int p = i >> 4, t = i & 15;  // maps past m0 have zero weights
+        k1[p][t] = make_float2(N->k1[2 * p][t], N->k1[2 * p + 1][t]);
     }
-    pool2[((long long)m * p2h + y) * p2w + x] = lg_pool_tanh(c, N->max_pool, N->cb[1][m], N->sw[1][m], N->sb[1][m], N->af);
+    for (int i = tid; i < m0 * 9; i += kLgT) k2[i / 9][i % 9] = make_float2(N->k2[2 * (i / 9)][i % 9], N->k2[2 * (i / 9) + 1][i % 9]);
+    if (tid < kLgMaxM0 / 2) q1[tid] = lg_pool_pair(*N, 0, tid);
+    if (tid < m0) q2[tid] = lg_pool_pair(*N, 1, tid);
+    const f2_t af = f2_dup(N->af);
+    const LgTable::Level& V = lg_level<&LgTable::Level::pool_base>(T, blockIdx.x);
+    const int tile = blockIdx.x - V.pool_base, ty = tile / V.pool_tx;
+    const int x0 = (tile - ty * V.pool_tx) * kLgTX, y0 = ty * kLgTY;
+    // of the L1 pixels, those that a pooled L2 pixel of the level reads
+    const int nx = min(kLgP1X, 2 * (V.p2w - x0) + 2), ny = min(kLgP1Y, 2 * (V.p2h - y0) + 2);
+    __syncthreads();
+    for (int it = tid; it < kLgP1X * ny; it += kLgT) {
+        const int y = it / kLgP1X, x = it - y * kLgP1X;
+        if (x >= nx) continue;
+        const float* src = V.L.img + (size_t)(2 * (2 * y0 + y)) * V.L.pitch + 2 * (2 * x0 + x);
+        f2_t win[5][5];
+#pragma unroll
+        for (int r = 0; r < 5; ++r)
+#pragma unroll
+            for (int c = 0; c < 5; ++c) win[r][c] = f2_dup(__ldg(src + (size_t)r * V.L.pitch + c));
+        float P[kLgMaxM0];
+#pragma unroll
+        for (int p = 0; p < kLgMaxM0 / 2; ++p) {
+            P[2 * p] = P[2 * p + 1] = 0.f;
+            if (2 * p >= m0) continue;
+            f2_t c[4];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const f2_t w = f2_ld(k1[p][t]);
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const f2_t m = f2_mul(win[(d >> 1) + (t >> 2)][(d & 1) + (t & 3)], w, nz);
+                    c[d] = t ? f2_add(c[d], m) : m;
+                }
+            }
+            const f2_t v = lg_pool_tanh2(c, max_pool, q1[p], af, nz);
+            P[2 * p] = f2_lo(v);
+            P[2 * p + 1] = f2_hi(v);
+        }
+#pragma unroll
+        for (int k = 0; k < kLgMaxM0; ++k)
+            if (k < m0) s1[k][y][x] = lg_neighbour_sum(P, k, m0);
+    }
+    __syncthreads();
+    const int lx = tid & (kLgTX - 1), ly = tid / kLgTX;
+    if (x0 + lx >= V.p2w || y0 + ly >= V.p2h) return;
+    float P[kLgMaxM1];
+#pragma unroll
+    for (int i = 0; i < kLgMaxM0; ++i) {
+        P[2 * i] = P[2 * i + 1] = 0.f;
+        if (i >= m0) continue;
+        f2_t q[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) q[r][c] = f2_dup(s1[i][2 * ly + r][2 * lx + c]);
+        f2_t c[4];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            const f2_t w = f2_ld(k2[i][t]);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                const f2_t m = f2_mul(q[(d >> 1) + t / 3][(d & 1) + t % 3], w, nz);
+                c[d] = t ? f2_add(c[d], m) : m;
+            }
+        }
+        const f2_t v = lg_pool_tanh2(c, max_pool, q2[i], af, nz);
+        P[2 * i] = f2_lo(v);
+        P[2 * i + 1] = f2_hi(v);
+    }
+    const size_t plane = (size_t)V.p2w * V.p2h;
+    float* out = V.L.scratch + (size_t)(y0 + ly) * V.p2w + x0 + lx;
+#pragma unroll
+    for (int k = 0; k < kLgMaxM1; ++k)
+        if (k < 2 * m0) out[k * plane] = lg_neighbour_sum(P, k, 2 * m0);
 }
 
-__global__ void legacy_out_kernel(const LegacyNet* __restrict__ Np, const float* __restrict__ pool2, int p2w, int p2h, int ow, int oh,
-                                  float* __restrict__ resp, int* __restrict__ counts, int chunk_base, float thr) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= ow || y >= oh) return;
-    const LegacyNet& N = *Np;
-    const long long plane = (long long)p2w * p2h;
-    const int it2 = N.m2 >> 1, kw = N.k3w;
-    float vals[kLgMaxM2];
-    float acc = 0.f;
-    for (int i = 0; i < it2; ++i) {
-        const auto in = [&](int t) { return lg_map_sum(pool2, plane, N.m1, i, (long long)(y + t / kw) * p2w + x + t % kw); };
-        const float v0 = lg_l3_value(N, 2 * i, in), v1 = lg_l3_value(N, 2 * i + 1, in);
-        if (N.full_connect) {
-            vals[2 * i] = v0;
-            vals[2 * i + 1] = v1;
-        } else {
-            const float pair = fadd(v1, v0);
-            acc = (i == 0) ? pair : fadd(acc, pair);
+// L3 maps (2i, 2i + 1) of 32 x 8 responses, a lane a column, on the sums of map i: every input row is
+// loaded once and continues the chains of the rows that it reaches (each output's taps stay in row-major
+// order); the pair's weights are in registers. done(row, (c0, c1)) takes each result.
+template <int KW, int KH, class Done>
+__device__ __forceinline__ void lg_l3_rows(const LegacyNet& N, int i, const float* __restrict__ in, int pitch, int last, f2_t nz, Done done) {
+    f2_t w[KH * KW];
+#pragma unroll
+    for (int t = 0; t < KH * KW; ++t) w[t] = f2_pack(__ldg(&N.k3[2 * i][t]), __ldg(&N.k3[2 * i + 1][t]));
+    f2_t acc[kLgTY];
+#pragma unroll
+    for (int r = 0; r < kLgTY + KH - 1; ++r) {
+        const float* row = in + (size_t)min(r, last) * pitch;  // rows past the map feed responses past it
+        f2_t v[KW];
+#pragma unroll
+        for (int c = 0; c < KW; ++c) v[c] = f2_dup(__ldg(row + c));
+#pragma unroll
+        for (int j = 0; j < kLgTY; ++j) {
+            const int kr = r - j;
+            if (kr < 0 || kr >= KH) continue;
+#pragma unroll
+            for (int c = 0; c < KW; ++c) {
+                const f2_t m = f2_mul(v[c], w[kr * KW + c], nz);
+                acc[j] = kr + c ? f2_add(acc[j], m) : m;
+            }
+            if (kr == KH - 1) done(j, acc[j]);
         }
     }
-    if (N.full_connect)
+}
+
+// L3 to the output of one 32 x 8 tile of responses: a warp takes every eighth map pair for the whole tile,
+// then a thread a response sums what the pairs left in shared memory, in map (or neuron) order.
+template <int KW, int KH>
+__global__ void __launch_bounds__(kLgT) legacy_out_kernel(const LegacyNet* __restrict__ Np, const __grid_constant__ LgTable T, int* __restrict__ counts,
+                                                          float thr, const f2_t nz) {
+    __shared__ float vals[kLgMaxM2][kLgTY][kLgTX];  // L3 values, or without a fully connected layer each pair's sum
+    const LegacyNet& N = *Np;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int it2 = N.m2 >> 1;
+    const LgTable::Level& V = lg_level<&LgTable::Level::out_base>(T, blockIdx.x);
+    const int tile = blockIdx.x - V.out_base, ty = tile / V.out_tx;
+    const int x0 = (tile - ty * V.out_tx) * kLgTX, y0 = ty * kLgTY;
+    const size_t plane = (size_t)V.p2w * V.p2h;
+    const int sx = min(x0 + lane, V.ow - 1);  // columns past the map compute the last one again
+    for (int i = warp; i < it2; i += kLgT / 32) {
+        const LgL3Pair q = lg_l3_pair(N, i);
+        const float* in = V.L.scratch + i * plane + (size_t)y0 * V.p2w + sx;
+        auto done = [&](int j, f2_t c) {
+            const f2_t v = lg_l3_finish2(N, q, c, nz);
+            if (N.full_connect) {
+                vals[2 * i][j][lane] = f2_lo(v);
+                vals[2 * i + 1][j][lane] = f2_hi(v);
+            } else {
+                vals[i][j][lane] = fadd(f2_hi(v), f2_lo(v));
+            }
+        };
+        if constexpr (KW > 0) {
+            lg_l3_rows<KW, KH>(N, i, in, V.p2w, V.p2h - 1 - y0, nz, done);
+        } else {
+            // any other kernel shape of the format: one output after the other
+            const int kw = N.k3w, kt = N.k3w * N.k3h;
+            for (int j = 0; j < kLgTY && y0 + j < V.oh; ++j) {
+                f2_t acc = 0ull;
+                for (int t = 0; t < kt; ++t) {
+                    const f2_t m = f2_mul(f2_dup(__ldg(in + (size_t)(j + t / kw) * V.p2w + t % kw)), f2_pack(N.k3[2 * i][t], N.k3[2 * i + 1][t]), nz);
+                    acc = t ? f2_add(acc, m) : m;
+                }
+                done(j, acc);
+            }
+        }
+    }
+    __syncthreads();
+    const int x = x0 + lane, y = y0 + warp;
+    if (x >= V.ow || y >= V.oh) return;
+    float acc = 0.f;
+    if (N.full_connect) {
         for (int n = 0; n < N.hl; ++n) {
-            const float h = lg_hidden_fc(N, n, vals);
+            const float h = lg_hidden_fc(N, n, [&](int j) { return vals[j][warp][lane]; });
             acc = (n == 0) ? h : fadd(acc, h);
         }
+    } else {
+        acc = vals[0][warp][lane];
+        for (int i = 1; i < it2; ++i) acc = fadd(acc, vals[i][warp][lane]);
+    }
     const float r = lg_finish(N, acc);
-    resp[(long long)y * ow + x] = r;
+    V.L.resp[(long long)y * V.ow + x] = r;
     // candidates (response > treshold_1) counted per scan chunk, as the CNTK stage-1 back kernel does
-    if (counts && r > thr) atomicAdd(&counts[chunk_base + (y * ow + x) / kCandChunk], 1);
+    if (counts && r > thr) atomicAdd(&counts[V.L.chunk_base + (y * V.ow + x) / kCandChunk], 1);
 }
 
 }  // namespace
 
-cudaError_t launch_legacy_forward(const LegacyNet* d_net, const LegacyNet& h_net, const float* img, int pitch, int w, int h, float* scratch,
-                                  float* resp, cudaStream_t st, int* counts, int chunk_base, float thr) {
-    const int p1w = (w - 3) >> 1, p1h = (h - 3) >> 1;
-    const int p2w = (((w - 3) >> 1) - 2) >> 1, p2h = (((h - 3) >> 1) - 2) >> 1;
-    int ow, oh;
-    legacy_output_size(h_net, w, h, &ow, &oh);
-    float* pool1 = scratch;
-    float* pool2 = scratch + (size_t)h_net.m0 * p1w * p1h;
-    const dim3 b(32, 8);
-    legacy_l1_kernel<<<dim3((p1w + 31) / 32, (p1h + 7) / 8, h_net.m0), b, 0, st>>>(d_net, img, pitch, p1w, p1h, pool1);
-    legacy_l2_kernel<<<dim3((p2w + 31) / 32, (p2h + 7) / 8, h_net.m1), b, 0, st>>>(d_net, pool1, p1w, p1h, p2w, p2h, pool2);
-    if (ow > 0 && oh > 0) legacy_out_kernel<<<dim3((ow + 31) / 32, (oh + 7) / 8), b, 0, st>>>(d_net, pool2, p2w, p2h, ow, oh, resp, counts, chunk_base, thr);
+// Two launches for up to kLgLevels levels. Before, every level took three (one thread a pooled pixel and map,
+// or a response with all its maps, each tap summing three maps from memory): the 13 levels of a 640 x 480
+// frame took 1.03 ms of kernels on B200, now 33 us (19 for L1 and L2, 14 for the rest).
+cudaError_t launch_legacy_forward(const LegacyNet* d_net, const LegacyNet& h_net, const LegacyLevel* levels, int n_levels, cudaStream_t st, int* counts,
+                                  float thr) {
+    const f2_t nz = 0x8000000080000000ull;  // (-0, -0)
+    for (int g0 = 0; g0 < n_levels; g0 += kLgLevels) {
+        LgTable T;
+        T.n = n_levels - g0 < kLgLevels ? n_levels - g0 : kLgLevels;
+        int pool = 0, out = 0;
+        for (int i = 0; i < T.n; ++i) {
+            LgTable::Level& V = T.lv[i];
+            V.L = levels[g0 + i];
+            V.p2w = (((V.L.w - 3) >> 1) - 2) >> 1;
+            V.p2h = (((V.L.h - 3) >> 1) - 2) >> 1;
+            legacy_output_size(h_net, V.L.w, V.L.h, &V.ow, &V.oh);
+            const bool any = V.ow > 0 && V.oh > 0;
+            V.pool_tx = (V.p2w + kLgTX - 1) / kLgTX;
+            V.pool_base = pool;
+            if (any) pool += V.pool_tx * ((V.p2h + kLgTY - 1) / kLgTY);
+            V.out_tx = (V.ow + kLgTX - 1) / kLgTX;
+            V.out_base = out;
+            if (any) out += V.out_tx * ((V.oh + kLgTY - 1) / kLgTY);
+        }
+        if (!pool) continue;
+        legacy_pool_kernel<<<pool, kLgT, 0, st>>>(d_net, T, nz);
+        if (h_net.k3w == 5 && h_net.k3h == 6)
+            legacy_out_kernel<5, 6><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
+        else if (h_net.k3w == 7 && h_net.k3h == 8)
+            legacy_out_kernel<7, 8><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
+        else
+            legacy_out_kernel<0, 0><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
+    }
     return cudaGetLastError();
 }
 
 size_t legacy_scratch_floats(const LegacyNet& n, int w, int h) {
-    const size_t p1 = (size_t)((w - 3) >> 1) * ((h - 3) >> 1);
-    const size_t p2 = (size_t)((((w - 3) >> 1) - 2) >> 1) * ((((h - 3) >> 1) - 2) >> 1);
-    return (size_t)n.m0 * p1 + (size_t)n.m1 * p2;
+    return (size_t)n.m1 * ((((w - 3) >> 1) - 2) >> 1) * ((((h - 3) >> 1) - 2) >> 1);
 }
 
 }  // namespace ccnn
@@ -287,9 +435,8 @@ extern "C" CCNN_API ccnn_status ccnn_legacy_net_forward(const char* model_path, 
     const size_t scratch = legacy_scratch_floats(net, cols, rows);
     cudaError_t e = cudaMallocAsync(&buf, sizeof(LegacyNet) + sizeof(float) * scratch, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(buf, &net, sizeof(LegacyNet), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = launch_legacy_forward((const LegacyNet*)buf, net, d_img, (int)(step / sizeof(float)), cols, rows,
-                                  (float*)((char*)buf + sizeof(LegacyNet)), d_resp, st, nullptr, 0, 0.f);
+    const LegacyLevel L = {d_img, (int)(step / sizeof(float)), cols, rows, (float*)((char*)buf + sizeof(LegacyNet)), d_resp, 0};
+    if (e == cudaSuccess) e = launch_legacy_forward((const LegacyNet*)buf, net, &L, 1, st, nullptr, 0.f);
     if (buf) {
         const cudaError_t f = cudaFreeAsync(buf, st);
         if (e == cudaSuccess) e = f;

@@ -188,64 +188,118 @@ __device__ void window_net(const NW& W, WindowSmem& S, int mode) {
     __syncthreads();
 }
 
-// The legacy (format 1.0) stage-2/3 networks on the window in shared memory: L1 (6 maps, 22x24
-// pooled) in S.s1, L2 (12 maps, 10x11) in S.p2, the L3 values of the 16 outputs in S.a3, fully
-// connected hidden neurons in S.hbuf; the arithmetic of the standalone legacy forward pass
-// (legacy_dev.cuh), spread over the block.
-__device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode) {
-    constexpr int kP1 = kP1W * kP1H, kP2 = kP2W * kP2H;
-    constexpr long long kS1Plane = kP1H * (kP1W + 1), kP2Plane = kP2H * (kP2W + 1);
-    for (int it = threadIdx.x; it < W.m0 * kP1; it += kWT) {
-        const int m = it / kP1, p = it - m * kP1;
-        const int x = p % kP1W, y = p / kP1W;
-        const float* k = W.k1[m];
-        float c[4];
+// The legacy (format 1.0) stage-2/3 networks on the window in shared memory: the sums of neighbouring L1 maps
+// (6 maps, 22x24 pooled) in S.s1, L2 (12 maps, 10x11) in S.p2 and their sums in S.s2, the L3 values of the
+// 16 outputs in S.a3, fully connected hidden neurons in S.hbuf; the arithmetic of the standalone legacy
+// forward pass (legacy_dev.cuh), map pairs packed, spread over the block. As in window_net, whole passes of
+// L1 pixels take every map pair a thread and the pixels of the last, partial pass one pair a warp. The windows
+// of a 640 x 480 frame took 81 us on B200 with one map a thread and the map sums made tap by tap, now 40.
+__device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f2_t nz) {
+    constexpr int kP2 = kP2W * kP2H;
+    constexpr int kM0 = 6;  // the most first-layer maps of a stage-2/3 network
+    constexpr int kFull = (kP1W * kP1H / kWT) * kWT, kRest = kP1W * kP1H - kFull, kMP = kM0 / 2;
+    static_assert(kRest > 0 && kRest <= 32 && 32 * kMP <= kWT, "partial L1 pass must fit one warp per map pair");
+    const int m0 = W.m0;
+    const f2_t af = f2_dup(W.af);
+    auto sums = [&](const float (&P)[kM0], int px) {
+        const int x = px % kP1W, y = px / kP1W;
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const int x0 = 2 * x + (d & 1), y0 = 2 * y + (d >> 1);
-            float acc = fmul(win_in(S, mode, x0, y0), k[0]);
+        for (int k = 0; k < kM0; ++k)
+            if (k < m0) S.s1[k][y][x] = lg_neighbour_sum(P, k, m0);
+    };
+    for (int p = threadIdx.x; p < kFull + 32 * kMP; p += kWT) {
+        const bool unit = p >= kFull;  // one map pair (warp-uniform) of a pixel of the partial pass
+        if (unit && ((p - kFull) & 31) >= kRest) continue;
+        const int px = unit ? kFull + ((p - kFull) & 31) : p;
+        const int mp0 = unit ? (p - kFull) >> 5 : 0;
+        const int x = px % kP1W, y = px / kP1W;
+        f2_t win[5][5];
 #pragma unroll
-            for (int t = 1; t < 16; ++t) acc = fadd(acc, fmul(win_in(S, mode, x0 + (t & 3), y0 + (t >> 2)), k[t]));
-            c[d] = acc;
+        for (int r = 0; r < 5; ++r)
+#pragma unroll
+            for (int c = 0; c < 5; ++c) win[r][c] = f2_dup(win_in(S, mode, 2 * x + c, 2 * y + r));
+        float P[kM0];
+#pragma unroll
+        for (int mp = 0; mp < kMP; ++mp) {
+            P[2 * mp] = P[2 * mp + 1] = 0.f;
+            if (2 * mp >= m0 || (unit && mp != mp0)) continue;
+            f2_t c[4];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const f2_t w = f2_pack(__ldg(&W.k1[2 * mp][t]), __ldg(&W.k1[2 * mp + 1][t]));
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const f2_t m = f2_mul(win[(d >> 1) + (t >> 2)][(d & 1) + (t & 3)], w, nz);
+                    c[d] = t ? f2_add(c[d], m) : m;
+                }
+            }
+            const f2_t v = lg_pool_tanh2(c, W.max_pool, lg_pool_pair(W, 0, mp), af, nz);
+            P[2 * mp] = f2_lo(v);
+            P[2 * mp + 1] = f2_hi(v);
+            if (unit) {
+                S.l1rest[px - kFull][2 * mp] = P[2 * mp];
+                S.l1rest[px - kFull][2 * mp + 1] = P[2 * mp + 1];
+            }
         }
-        S.s1[m][y][x] = lg_pool_tanh(c, W.max_pool, W.cb[0][m], W.sw[0][m], W.sb[0][m], W.af);
+        if (!unit) sums(P, px);
     }
     __syncthreads();
-    const float* s1 = &S.s1[0][0][0];
-    for (int it = threadIdx.x; it < W.m1 * kP2; it += kWT) {
-        const int m = it / kP2, p = it - m * kP2;
-        const int x = p % kP2W, y = p / kP2W, i = m >> 1;
-        float Q[4][4];
+    if (threadIdx.x < kRest) {
+        float P[kM0];
+#pragma unroll
+        for (int k = 0; k < kM0; ++k) P[k] = S.l1rest[threadIdx.x][k];
+        sums(P, kFull + threadIdx.x);
+    }
+    __syncthreads();
+    for (int it = threadIdx.x; it < m0 * kP2; it += kWT) {
+        const int i = it / kP2, p = it - i * kP2;
+        const int x = p % kP2W, y = p / kP2W;
+        f2_t q[4][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) Q[r][q] = lg_map_sum(s1, kS1Plane, W.m0, i, (2 * y + r) * (kP1W + 1) + 2 * x + q);
-        const float* k = W.k2[m];
-        float c[4];
+            for (int c = 0; c < 4; ++c) q[r][c] = f2_dup(S.s1[i][2 * y + r][2 * x + c]);
+        f2_t c[4];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const int dy = d >> 1, dx = d & 1;
-            float acc = fmul(Q[dy][dx], k[0]);
+        for (int t = 0; t < 9; ++t) {
+            const f2_t w = f2_pack(__ldg(&W.k2[2 * i][t]), __ldg(&W.k2[2 * i + 1][t]));
 #pragma unroll
-            for (int t = 1; t < 9; ++t) acc = fadd(acc, fmul(Q[dy + t / 3][dx + t % 3], k[t]));
-            c[d] = acc;
+            for (int d = 0; d < 4; ++d) {
+                const f2_t m = f2_mul(q[(d >> 1) + t / 3][(d & 1) + t % 3], w, nz);
+                c[d] = t ? f2_add(c[d], m) : m;
+            }
         }
-        S.p2[m][y][x] = lg_pool_tanh(c, W.max_pool, W.cb[1][m], W.sw[1][m], W.sb[1][m], W.af);
+        const f2_t v = lg_pool_tanh2(c, W.max_pool, lg_pool_pair(W, 1, i), af, nz);
+        S.p2[2 * i][y][x] = f2_lo(v);
+        S.p2[2 * i + 1][y][x] = f2_hi(v);
     }
     __syncthreads();
-    const float* p2 = &S.p2[0][0][0];
-    for (int it = threadIdx.x; it < W.m2 * kOutN; it += kWT) {
-        const int m = it / kOutN, o = it - m * kOutN;
-        const int ox = o & 3, oy = o >> 2, i = m >> 1, kw = W.k3w;
-        S.a3[m][o] = lg_l3_value(W, m, [&](int t) { return lg_map_sum(p2, kP2Plane, W.m1, i, (oy + t / kw) * (kP2W + 1) + ox + t % kw); });
+    for (int it = threadIdx.x; it < W.m1 * kP2; it += kWT) {
+        const int k = it / kP2, p = it - k * kP2;
+        const int x = p % kP2W, y = p / kP2W;
+        const float two = k ? fadd(S.p2[k - 1][y][x], S.p2[k][y][x]) : fadd(S.p2[0][y][x], S.p2[1][y][x]);
+        S.s2[k][y][x] = (k == 0 || k == W.m1 - 1) ? two : fadd(two, S.p2[k + 1][y][x]);
+    }
+    __syncthreads();
+    constexpr int kK3W = 7, kK3H = 8;  // the third-layer kernel of the stage-2/3 networks
+    for (int it = threadIdx.x; it < (W.m2 >> 1) * kOutN; it += kWT) {
+        const int i = it / kOutN, o = it - i * kOutN;
+        const int ox = o & 3, oy = o >> 2;
+        f2_t acc = 0ull;
+#pragma unroll
+        for (int t = 0; t < kK3W * kK3H; ++t) {
+            const f2_t m = f2_mul(f2_dup(S.s2[i][oy + t / kK3W][ox + t % kK3W]), f2_pack(__ldg(&W.k3[2 * i][t]), __ldg(&W.k3[2 * i + 1][t])), nz);
+            acc = t ? f2_add(acc, m) : m;
+        }
+        const f2_t v = lg_l3_finish2(W, lg_l3_pair(W, i), acc, nz);
+        S.a3[2 * i][o] = f2_lo(v);
+        S.a3[2 * i + 1][o] = f2_hi(v);
     }
     __syncthreads();
     if (W.full_connect) {
         for (int it = threadIdx.x; it < W.hl * kOutN; it += kWT) {
             const int n = it / kOutN, o = it - n * kOutN;
-            float vals[kLgMaxM2];
-            for (int j = 0; j < W.m2; ++j) vals[j] = S.a3[j][o];
-            S.hbuf[n][o] = lg_hidden_fc(W, n, vals);
+            S.hbuf[n][o] = lg_hidden_fc(W, n, [&](int j) { return S.a3[j][o]; });
         }
         __syncthreads();
     }
@@ -273,6 +327,7 @@ struct WinArgs {
     WinOut* out;
     CascadeConfig cfg;
     const LegacyNet* lg;  // legacy networks ([1] stage 2, [2] stage 3) instead of the CNTK ones, or null
+    float2 negzero;       // (-0, -0), for the legacy networks (the CNTK ones carry their own)
 };
 
 // crop + byte rounding + (optional) equalisation of one window into S.crop
@@ -382,7 +437,7 @@ __device__ __forceinline__ void window_item(const WindowNets& N, const WinArgs& 
     r[1].knn = 0;
     for (int stage = 0; stage < 2; ++stage) {
         if constexpr (kLegacy)
-            legacy_window_net(a.lg[1 + stage], S, stage == 0 ? 0 : (C.reflection ? 1 : 2));
+            legacy_window_net(a.lg[1 + stage], S, stage == 0 ? 0 : (C.reflection ? 1 : 2), f2_ld(a.negzero));
         else if (stage == 0)
             window_net(N.s2, S, 0);
         else
@@ -487,7 +542,10 @@ cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, in
     a.out = out;
     a.cfg = cfg;
     a.lg = lg;
-    if (lg)
+    a.negzero = make_float2(-0.f, -0.f);
+    if (lg && ctas_per_sm <= 2)
+        window_kernel<true, 2><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
+    else if (lg)
         window_kernel<true, 4><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
     else if (ctas_per_sm <= 2)
         window_kernel<false, 2><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);

@@ -202,10 +202,18 @@ cudaError_t window_setup();
 cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, int gw, int gh, const Candidate* cands, const int* n_cand,
                           const LevelDesc* levels, WinOut* out, const CascadeConfig& cfg, int grid, cudaStream_t st,
                           const LegacyNet* lg = nullptr, int ctas_per_sm = 4);
-// one legacy (format 1.0) network on a w x h image (pitch floats): scratch holds its pooled L1 and
-// L2 maps; counts (optional) gets each scan chunk's responses above thr
-cudaError_t launch_legacy_forward(const LegacyNet* d_net, const LegacyNet& h_net, const float* img, int pitch, int w, int h, float* scratch,
-                                  float* resp, cudaStream_t st, int* counts, int chunk_base, float thr);
+// one legacy (format 1.0) network on each of the levels; counts (optional) gets each scan chunk's responses
+// above thr
+struct LegacyLevel {
+    const float* img;
+    int pitch, w, h;  // pitch in floats
+    float* scratch;   // legacy_scratch_floats: the sums of neighbouring pooled L2 maps
+    float* resp;      // dense, legacy_output_size
+    int chunk_base;
+};
+size_t legacy_scratch_floats(const LegacyNet& n, int w, int h);
+cudaError_t launch_legacy_forward(const LegacyNet* d_net, const LegacyNet& h_net, const LegacyLevel* levels, int n_levels, cudaStream_t st, int* counts,
+                                  float thr);
 int window_smem_bytes();
 // facial analysis: dynamic shared memory attribute (once per device) and the landmark kernel
 cudaError_t facial_setup();
