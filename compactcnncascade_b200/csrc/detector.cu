@@ -761,6 +761,9 @@ ReplayArgs Detector::replay_args(Slot& s, const Plan& p) const {
     a.n_faces = s.d_nfaces;
     a.m_out = s.d_mk;
     a.n_m_out = s.d_nmk;
+    a.host_faces = s.h_faces;
+    a.host_n_faces = s.h_nfaces;
+    a.host_cap = kHostFaces;
     return a;
 }
 
@@ -801,23 +804,20 @@ ccnn_status Detector::enqueue_kernels(Slot& s, const Plan& p) {
         CCNN_CUDA(cudaMemsetAsync(s.d_sync1, 0, sizeof(int) * (2 + kBatchStages), s.st));
         CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, s.d_sync1, s.d_sync1 + 1 + kBatchStages,
                                       sm_count_ * stage1_batch_blocks_per_sm(batch_bpsm_), s.st));
-        CCNN_CUDA(cudaMemcpyAsync(s.h_nfaces + 1, s.d_sync1 + 1 + kBatchStages, sizeof(int), cudaMemcpyDeviceToHost, s.st));
     } else {
-        // the legacy network reads stored level images; the CNTK front kernel resamples its tiles from
-        // the gray frame itself
-        if (legacy_) CCNN_CUDA(launch_pyramid(p.levels.data(), p.n_levels, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_limg, s.st));
-        // the back kernel counts each chunk's candidates as it writes the responses
-        if (!p.chunks.empty()) CCNN_CUDA(cudaMemsetAsync(s.d_counts, 0, sizeof(int) * p.chunks.size(), s.st));
-    }
-    if (!single) {
+        // the back kernel counts each chunk's candidates as it writes the responses (from zero: the front
+        // kernel's first block clears them). The legacy network reads stored level images; the CNTK front
+        // kernel resamples its tiles from the gray frame itself
         if (legacy_) {
+            if (!p.chunks.empty()) CCNN_CUDA(cudaMemsetAsync(s.d_counts, 0, sizeof(int) * p.chunks.size(), s.st));
+            CCNN_CUDA(launch_pyramid(p.levels.data(), p.n_levels, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_limg, s.st));
             const ccnn_status ls = enqueue_legacy_stage1(s, p);
             if (ls != CCNN_OK) return ls;
         } else {
             CCNN_CUDA(launch_stage1(w1_, p.levels.data(), p.n_levels, nullptr, s.d_s1, s.d_resp, s.st, s.d_counts, cfg_.thr1,
                                     gated ? s.d_front_on : nullptr, gated ? s.d_back_on : nullptr,
                                     gated ? gate_cells(s.gate, p.gw, p.gh, gate_amb_frac_, gate_margin_) : GateCells{}, s1_sched_,
-                                    GrayRef{s.d_gray, s.gray_pitch, p.gw, p.gh}));
+                                    GrayRef{s.d_gray, s.gray_pitch, p.gw, p.gh}, (int)p.chunks.size()));
         }
     }
     CCNN_CUDA(launch_cand_write(p.d_chunks, (int)p.chunks.size(), p.d_levels, s.d_resp, cfg_.thr1, s.d_counts, s.d_cands, s.d_ncand,
@@ -829,8 +829,7 @@ ccnn_status Detector::enqueue_kernels(Slot& s, const Plan& p) {
         CCNN_CUDA(launch_facial(d_lnet_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_, s.d_attr,
                                 facial_grid_, s.st));
     CCNN_CUDA(launch_replay(replay_args(s, p), s.st));
-    CCNN_CUDA(cudaMemcpyAsync(s.h_nfaces, s.d_nfaces, sizeof(int), cudaMemcpyDeviceToHost, s.st));
-    CCNN_CUDA(cudaMemcpyAsync(s.h_faces, s.d_faces, sizeof(FaceOut) * kGraphFaces, cudaMemcpyDeviceToHost, s.st));
+    if (single) CCNN_CUDA(cudaMemcpyAsync(s.h_nfaces + 1, s.d_sync1 + 1 + kBatchStages, sizeof(int), cudaMemcpyDeviceToHost, s.st));
     return CCNN_OK;
 }
 
@@ -928,8 +927,8 @@ ccnn_status Detector::enqueue(Slot& s, const Plan& p, const ccnn_image& img, boo
     return CCNN_OK;
 }
 
-// Waits for slot s's frame and returns its faces: the graph downloads the first kGraphFaces; more
-// (up to `cap`) are fetched here. *src points at `cap`-or-fewer FaceOut entries valid until the
+// Waits for slot s's frame and returns its faces: the replay kernel leaves the first kHostFaces in host
+// memory; more (up to `cap`) are fetched here. *src points at `cap`-or-fewer FaceOut entries valid until the
 // next call on the slot.
 ccnn_status Detector::collect_raw(Slot& s, int cap, int* n, const FaceOut** src) {
     CCNN_CUDA(cudaEventSynchronize(s.done));
@@ -943,15 +942,10 @@ ccnn_status Detector::collect_raw(Slot& s, int cap, int* n, const FaceOut** src)
     *n = nf;
     const int take = std::min(nf, cap);
     *src = s.h_faces;
-    if (take > kGraphFaces) {
-        if (take > kHostFaces) {
-            s.h_extra.resize(take);
-            CCNN_CUDA(cudaMemcpy(s.h_extra.data(), s.d_faces, sizeof(FaceOut) * take, cudaMemcpyDeviceToHost));
-            *src = s.h_extra.data();
-        } else {
-            CCNN_CUDA(cudaMemcpy(s.h_faces + kGraphFaces, s.d_faces + kGraphFaces, sizeof(FaceOut) * (take - kGraphFaces),
-                                 cudaMemcpyDeviceToHost));
-        }
+    if (take > kHostFaces) {
+        s.h_extra.resize(take);
+        CCNN_CUDA(cudaMemcpy(s.h_extra.data(), s.d_faces, sizeof(FaceOut) * take, cudaMemcpyDeviceToHost));
+        *src = s.h_extra.data();
     }
     return CCNN_OK;
 }
@@ -1708,6 +1702,7 @@ ccnn_status Detector::launch_batch(BatchCtx& c, const Plan& p, const ccnn_image*
             ra[f].faces = c.d_faces + (size_t)f * face_cap;
             ra[f].face_cap = (int)face_cap;
             ra[f].n_faces = c.d_nf + f;
+            ra[f].host_faces = nullptr;  // a group's results come back together
         }
         CCNN_CUDA(cudaMemcpyAsync(c.d_rargs, ra.data(), sizeof(ReplayArgs) * B, cudaMemcpyHostToDevice, st));
         CCNN_CUDA(cudaStreamSynchronize(st));

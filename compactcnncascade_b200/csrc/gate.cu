@@ -166,6 +166,7 @@ __global__ void gate_mask_kernel(const __grid_constant__ LevelTable LT, int nb, 
                                  int w16, int h16, int margin, const int* __restrict__ ambiguous, int amb_limit, uint8_t* __restrict__ back_on,
                                  uint8_t* __restrict__ front_on) {
     extern __shared__ uint32_t sbits[];
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const LevelDesc& last = LT.lv[LT.n - 1];
     const bool full = *ambiguous > amb_limit;
@@ -254,8 +255,9 @@ cudaError_t launch_gate(const GateNet& net, const float* gray, int gpitch, int g
         const int nb = last.k2_base + last.k2_tiles_x * ((last.oh + kK2TileY - 1) / kK2TileY) - T.lv[0].k2_base;
         const int nf = last.k1_base + last.k1_tiles_x * ((last.p1h + kK1TileY - 1) / kK1TileY) - T.lv[0].k1_base;
         if (nb + nf > 0)
-            gate_mask_kernel<<<blocks(nb + nf, 128), 128, n_words <= kMaskSmemWords ? sizeof(uint32_t) * n_words : 0, st>>>(
-                T, nb, sc.bits, n_words, wwords, w16, h16, margin, sc.ambiguous, amb_limit, back_on, front_on);
+            e = launch_chained(gate_mask_kernel, blocks(nb + nf, 128), 128, n_words <= kMaskSmemWords ? sizeof(uint32_t) * n_words : 0, st, T, nb, sc.bits,
+                               n_words, wwords, w16, h16, margin, sc.ambiguous, amb_limit, back_on, front_on);
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }

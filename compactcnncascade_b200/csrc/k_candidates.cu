@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kChunkThreads) cand_write_kernel(const int4* _
                                                                    const LevelDesc* __restrict__ levels, const float* __restrict__ resp,
                                                                    float thr, const int* __restrict__ counts, Candidate* __restrict__ out,
                                                                    int* __restrict__ n_out, int cap) {
+    chain_wait();
     cand_write_chunk(chunks, n_chunks, levels, resp, thr, counts, out, n_out, cap, blockIdx.x);
 }
 
@@ -118,8 +119,7 @@ cudaError_t launch_cand_write_batch(const int4* d_chunks, int n_chunks, const Le
 cudaError_t launch_cand_write(const int4* d_chunks, int n_chunks, const LevelDesc* d_levels, const float* resp, float thr,
                               const int* counts, Candidate* out, int* n_out, int cap, cudaStream_t st) {
     if (n_chunks <= 0) return cudaMemsetAsync(n_out, 0, sizeof(int), st);
-    cand_write_kernel<<<n_chunks, kChunkThreads, 0, st>>>(d_chunks, n_chunks, d_levels, resp, thr, counts, out, n_out, cap);
-    return cudaGetLastError();
+    return launch_chained(cand_write_kernel, n_chunks, kChunkThreads, 0, st, d_chunks, n_chunks, d_levels, resp, thr, counts, out, n_out, cap);
 }
 
 }  // namespace ccnn

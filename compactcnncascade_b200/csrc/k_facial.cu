@@ -167,6 +167,7 @@ struct FacialArgs {
 __global__ void __launch_bounds__(kFT, 1) facial_kernel(const FacialArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FacialSmem& S = *reinterpret_cast<FacialSmem*>(smem_raw);
+    chain_wait();
     const int n = *a.n_cand;
     for (int ci = blockIdx.x; ci < n; ci += gridDim.x) {
         if (threadIdx.x == 0) {
@@ -228,8 +229,7 @@ cudaError_t launch_facial(const LandmarkNet* d_net, const float* gray, int gpitc
     a.win = win;
     a.cfg = cfg;
     a.attr = attr;
-    facial_kernel<<<grid, kFT, sizeof(FacialSmem), st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(facial_kernel, grid, kFT, sizeof(FacialSmem), st, a);
 }
 
 }  // namespace ccnn

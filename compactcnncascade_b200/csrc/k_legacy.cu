@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(kLgT) legacy_pool_kernel(const LegacyNet* __re
     __shared__ float2 k1[kLgMaxM0 / 2][16], k2[kLgMaxM0][9];
     __shared__ LgPoolPair q1[kLgMaxM0 / 2], q2[kLgMaxM0];
     const int tid = threadIdx.x;
+    chain_wait();
     const int m0 = N->m0, max_pool = N->max_pool;
     for (int i = tid; i < kLgMaxM0 / 2 * 16; i += kLgT) {
         const int p = i >> 4, t = i & 15;  // maps past m0 have zero weights
@@ -293,6 +294,7 @@ template <int KW, int KH>
 __global__ void __launch_bounds__(kLgT) legacy_out_kernel(const LegacyNet* __restrict__ Np, const __grid_constant__ LgTable T, int* __restrict__ counts,
                                                           float thr, const f2_t nz) {
     __shared__ float vals[kLgMaxM2][kLgTY][kLgTX];  // L3 values, or without a fully connected layer each pair's sum
+    chain_wait();
     const LegacyNet& N = *Np;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int it2 = N.m2 >> 1;
@@ -374,15 +376,15 @@ cudaError_t launch_legacy_forward(const LegacyNet* d_net, const LegacyNet& h_net
             if (any) out += V.out_tx * ((V.oh + kLgTY - 1) / kLgTY);
         }
         if (!pool) continue;
-        legacy_pool_kernel<<<pool, kLgT, 0, st>>>(d_net, T, nz);
-        if (h_net.k3w == 5 && h_net.k3h == 6)
-            legacy_out_kernel<5, 6><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
-        else if (h_net.k3w == 7 && h_net.k3h == 8)
-            legacy_out_kernel<7, 8><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
-        else
-            legacy_out_kernel<0, 0><<<out, kLgT, 0, st>>>(d_net, T, counts, thr, nz);
+        cudaError_t e = launch_chained(legacy_pool_kernel, pool, kLgT, 0, st, d_net, T, nz);
+        if (e != cudaSuccess) return e;
+        const auto kernel = h_net.k3w == 5 && h_net.k3h == 6   ? legacy_out_kernel<5, 6>
+                            : h_net.k3w == 7 && h_net.k3h == 8 ? legacy_out_kernel<7, 8>
+                                                               : legacy_out_kernel<0, 0>;
+        e = launch_chained(kernel, out, kLgT, 0, st, d_net, T, counts, thr, nz);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 size_t legacy_scratch_floats(const LegacyNet& n, int w, int h) {

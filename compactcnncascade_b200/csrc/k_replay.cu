@@ -1094,6 +1094,15 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
         a.faces[i] = f;
     }
     if (tid == 0) *a.n_faces = nF;
+    if (a.host_faces) {
+        // the result straight into the caller's page-locked memory, a warp's stores side by side (two copies
+        // after the kernel took 5 us of a frame's latency)
+        __syncthreads();
+        constexpr int kWords = sizeof(FaceOut) / sizeof(int);
+        const int words = imin(imin(nF, a.face_cap), a.host_cap) * kWords;
+        for (int i = tid; i < words; i += kRT) reinterpret_cast<int*>(a.host_faces)[i] = reinterpret_cast<const int*>(a.faces)[i];
+        if (tid == 0) *a.host_n_faces = nF;
+    }
 }
 
 // Detect with the caller's detections in front (cnn_detector_v3.cpp:2753-2806), one warp: the
@@ -1145,7 +1154,10 @@ cudaError_t launch_nms(const Det* in, int n, uint8_t* checked, Det* out, int* n_
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kRT, 1) replay_kernel(const ReplayArgs a) { replay_body(a); }
+__global__ void __launch_bounds__(kRT, 1) replay_kernel(const ReplayArgs a) {
+    chain_wait();
+    replay_body(a);
+}
 
 // the frames of a batch: block f replays args[f]
 __global__ void __launch_bounds__(kRT, 1) replay_batch_kernel(const ReplayArgs* __restrict__ args) {
@@ -1198,8 +1210,7 @@ cudaError_t replay_setup() {
 }
 
 cudaError_t launch_replay(const ReplayArgs& a, cudaStream_t st) {
-    replay_kernel<<<1, kRT, kReplaySmemBytes, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(replay_kernel, 1, kRT, kReplaySmemBytes, st, a);
 }
 
 cudaError_t launch_replay_batch(const ReplayArgs* d_args, int n_frames, cudaStream_t st) {

@@ -347,8 +347,12 @@ __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const
 template <bool kFromGray, int kMinBlocks>
 __global__ void __launch_bounds__(kFrontThreads, kMinBlocks) stage1_front_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ LevelTable LT,
                                                               const float* __restrict__ limg, const GrayRef G, float* __restrict__ s1,
-                                                              const uint8_t* __restrict__ front_on, const GateCells cells) {
+                                                              const uint8_t* __restrict__ front_on, const GateCells cells, int* __restrict__ counts,
+                                                              int n_counts) {
     __shared__ FrontSmem S;
+    chain_wait();
+    if (blockIdx.x == 0)  // the back kernel's candidate counts start from zero
+        for (int i = threadIdx.x; i < n_counts; i += kFrontThreads) counts[i] = 0;
     const int g = LT.first + blockIdx.x;
     if (front_on && !front_on[g]) return;  // gated off: no back tile reads this one
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k1_base>(LT, g)];
@@ -655,6 +659,7 @@ __global__ void __launch_bounds__(256 / kPairs, kMinBlocks) stage1_back_kernel(c
     const int g = LT.first + blockIdx.x;
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k2_base>(LT, g)];
     const int t = g - L.k2_base;
+    chain_wait();
     back_tile<kPairs, false>(D, S, L, t, g, s1, resp, counts, thr, back_on, cells);
 }
 
@@ -705,24 +710,23 @@ static cudaError_t launch_grouped(const LevelDesc* levels, int n_levels, int Lev
         T.first = T.lv[0].*base;
         const LevelDesc& last = T.lv[T.n - 1];
         const int blocks = last.*base + tiles(last) - T.first;
-        if (blocks > 0) launch(T, blocks);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = blocks > 0 ? launch(T, blocks) : cudaSuccess;
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_stage1_front(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* limg, float* s1, cudaStream_t st,
-                                const uint8_t* front_on, Stage1Sched sched, GrayRef gray, GateCells cells) {
+                                const uint8_t* front_on, Stage1Sched sched, GrayRef gray, GateCells cells, int* counts, int n_counts) {
     return launch_grouped(
         levels, n_levels, &LevelDesc::k1_base, [](const LevelDesc& L) { return L.k1_tiles_x * ((L.p1h + kK1TileY - 1) / kK1TileY); },
         [&](const LevelTable& T, int blocks) {
             const bool six = sched.front_blocks_per_sm >= 4;
-            if (gray.p)
-                (six ? stage1_front_kernel<true, 6> : stage1_front_kernel<true, 5>)<<<blocks, kFrontThreads, 0, st>>>(W, T, limg, gray, s1, front_on, cells);
-            else
-                (six ? stage1_front_kernel<false, 6> : stage1_front_kernel<false, 5>)<<<blocks, kFrontThreads, 0, st>>>(W, T, limg, gray, s1, front_on,
-                                                                                                                         cells);
+            const auto kernel = gray.p ? (six ? stage1_front_kernel<true, 6> : stage1_front_kernel<true, 5>)
+                                       : (six ? stage1_front_kernel<false, 6> : stage1_front_kernel<false, 5>);
+            const cudaError_t e = launch_chained(kernel, blocks, kFrontThreads, 0, st, W, T, limg, gray, s1, front_on, cells, counts, n_counts);
+            n_counts = 0;  // by the first launch
+            return e;
         });
 }
 
@@ -742,18 +746,15 @@ cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_
     return launch_grouped(
         levels, n_levels, &LevelDesc::k2_base, [](const LevelDesc& L) { return L.k2_tiles_x * ((L.oh + kK2TileY - 1) / kK2TileY); },
         [&](const LevelTable& T, int blocks) {
-            if (two_pairs)
-                (sched.back_blocks_per_sm >= 4 ? stage1_back_kernel<2, 6> : stage1_back_kernel<2, 5>)<<<blocks, 128, 0, st>>>(D, T, s1, resp, counts, thr,
-                                                                                                                               back_on, cells);
-            else
-                stage1_back_kernel<1, 3><<<blocks, 256, 0, st>>>(D, T, s1, resp, counts, thr, back_on, cells);
+            const auto kernel = two_pairs ? (sched.back_blocks_per_sm >= 4 ? stage1_back_kernel<2, 6> : stage1_back_kernel<2, 5>) : stage1_back_kernel<1, 3>;
+            return launch_chained(kernel, blocks, two_pairs ? 128 : 256, 0, st, D, T, s1, resp, counts, thr, back_on, cells);
         });
 }
 
 cudaError_t launch_stage1(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* limg, float* s1, float* resp,
                           cudaStream_t st, int* counts, float thr, const uint8_t* front_on, const uint8_t* back_on, GateCells cells,
-                          Stage1Sched sched, GrayRef gray) {
-    cudaError_t e = launch_stage1_front(W, levels, n_levels, limg, s1, st, front_on, sched, gray, cells);
+                          Stage1Sched sched, GrayRef gray, int n_counts) {
+    cudaError_t e = launch_stage1_front(W, levels, n_levels, limg, s1, st, front_on, sched, gray, cells, counts, n_counts);
     if (e != cudaSuccess) return e;
     return launch_stage1_back(W, levels, n_levels, s1, resp, st, counts, thr, back_on, cells, sched);
 }

@@ -472,6 +472,7 @@ template <bool kLegacy, int kMinBlocks>
 __global__ void __launch_bounds__(kWT, kMinBlocks) window_kernel(const __grid_constant__ WindowNets N, const WinArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WindowSmem& S = *reinterpret_cast<WindowSmem*>(smem_raw);
+    chain_wait();
     const int n = *a.n_cand;
     const int per_cand = a.cfg.double_check ? 2 : 1;
     const int total = n * per_cand;
@@ -543,19 +544,12 @@ cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, in
     a.cfg = cfg;
     a.lg = lg;
     a.negzero = make_float2(-0.f, -0.f);
-    if (lg && ctas_per_sm <= 2)
-        window_kernel<true, 2><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    else if (lg)
-        window_kernel<true, 4><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    else if (ctas_per_sm <= 2)
-        window_kernel<false, 2><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    else if (ctas_per_sm == 5)
-        window_kernel<false, 5><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    else if (ctas_per_sm >= 6)
-        window_kernel<false, 6><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    else
-        window_kernel<false, 4><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a);
-    return cudaGetLastError();
+    const auto kernel = lg ? (ctas_per_sm <= 2 ? window_kernel<true, 2> : window_kernel<true, 4>)
+                        : ctas_per_sm <= 2 ? window_kernel<false, 2>
+                        : ctas_per_sm == 5 ? window_kernel<false, 5>
+                        : ctas_per_sm >= 6 ? window_kernel<false, 6>
+                                           : window_kernel<false, 4>;
+    return launch_chained(kernel, grid, kWT, sizeof(WindowSmem), st, N, a);
 }
 
 // five or six resident window blocks need most of a SM's 228 KB as shared memory

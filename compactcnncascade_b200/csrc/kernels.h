@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstdint>
+#include <utility>
+
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -9,6 +11,28 @@
 #include "legacy.h"
 
 namespace ccnn {
+
+#if defined(__CUDACC__)
+// The kernels of a frame's chain are launched as programmatic dependents: a kernel's blocks are set up while
+// the one before it in the stream ends, and wait here, before they touch memory, until it has ended and its
+// writes are visible. Every block of such a kernel waits, so that the wait covers all earlier kernels too.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+#endif
 
 struct FaceOut {
     int x, y, w, h;
@@ -48,6 +72,10 @@ struct ReplayArgs {
     // their count, for callers that merge them again with detections of their own
     Det* m_out;
     int* n_m_out;
+    // the frame's result in host memory (mapped, optional): the face count and the first host_cap faces
+    FaceOut* host_faces;
+    int* host_n_faces;
+    int host_cap;
 };
 
 // the gray kernel instantiation for `ch` channels, with or without the gate features (to find its
@@ -176,18 +204,19 @@ struct GrayRef {
 };
 // stage-1 net over all levels; `levels` is a HOST array (the descriptors travel as kernel
 // parameters); level tiles resampled from `gray`, or read from limg + img_off when gray.p is null
-// counts (optional, zeroed by the caller): per candidate-scan chunk, responses > thr
+// counts (optional): per candidate-scan chunk, responses > thr; the first n_counts of them are zeroed by the
+// front kernel (0: by the caller)
 // cells (optional): the gate's cell bitmaps; a response above thr whose window centre has no likely
 // cell within cells.margin cells of it (in its level's octave) is written below every threshold
 cudaError_t launch_stage1(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* limg, float* s1, float* resp,
                           cudaStream_t st, int* counts = nullptr, float thr = 0.f, const uint8_t* front_on = nullptr,
                           const uint8_t* back_on = nullptr, GateCells cells = GateCells{}, Stage1Sched sched = Stage1Sched{},
-                          GrayRef gray = GrayRef{});
+                          GrayRef gray = GrayRef{}, int n_counts = 0);
 // front_on / back_on (optional): per-tile activity from the gate; inactive back tiles write
 // responses below every threshold
 cudaError_t launch_stage1_front(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* limg, float* s1, cudaStream_t st,
                                 const uint8_t* front_on = nullptr, Stage1Sched sched = Stage1Sched{}, GrayRef gray = GrayRef{},
-                                GateCells cells = GateCells{});
+                                GateCells cells = GateCells{}, int* counts = nullptr, int n_counts = 0);
 // shared-memory carve-out of the stage-1 back kernels (once per device before any launch)
 cudaError_t stage1_setup();
 cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_levels, const float* s1, float* resp, cudaStream_t st,
