@@ -166,7 +166,7 @@ struct NetWeights {
     static constexpr int kM1 = M1, kM2 = M2, kM3 = M3;
     static constexpr int kK1W = K1W, kK1H = K1H, kK2W = K2W, kK2H = K2H, kK3W = K3W, kK3H = K3H;
     static constexpr int kHL = HL, kConn = CONN, kHS = HS, kGroups = HL / HS;
-    float2 k1d[M1][K1W * K1H];      // L1 taps duplicated (w, w): two pixels of one map per packed op
+    alignas(16) float2 k1d[M1][K1W * K1H];  // L1 taps duplicated (w, w): two pixels of one map per packed op
     float2 k1p[M1 / 2][K1W * K1H];  // L1 taps of maps (2i, 2i+1), which read the same input
     float b1[M1], w1a[M1], w1b[M1], bn1[M1];
     float2 a1d[M1][4];              // L1 {b, w1a, w1b, bn} of each map duplicated (v, v)
@@ -174,7 +174,7 @@ struct NetWeights {
     float2 k2p[M2 / 2][K2W * K2H];  // L2 taps of maps (2i, 2i+1), which read the same sum map i
     float b2[M2], w2a[M2], w2b[M2], bn2[M2];
     float2 a2p[M2 / 2][4];          // L2 {b, w2a, w2b, bn} of map pairs
-    float2 k3p[M3 / 2][K3W * K3H];  // L3 taps of maps (2i, 2i+1)
+    alignas(16) float2 k3p[M3 / 2][K3W * K3H];  // L3 taps of maps (2i, 2i+1)
     float b3[M3], w3a[M3], w3b[M3], bn3[M3];
     float2 a3p[M3 / 2][4];          // L3 {b, w3a, w3b, bn} of map pairs
     float2 hwp[HL / 2][CONN];       // hidden weights of neurons (2q, 2q+1); neuron n = HS*i + t reads
@@ -230,13 +230,15 @@ struct LandmarkNet {
     float2 a1p[kM1 / 2][4];         // L1 {b, w1a, w1b, bn} of map pairs
     float2 k2p[kM2 / 2][9];         // L2 maps (2i, 2i+1) read neighbour sum i
     float2 a2p[kM2 / 2][4];
-    float2 k3p[kM3 / 2][kK3W * kK3H];  // L3 maps (2i, 2i+1) read neighbour sum i
+    // L3 and the hidden layer run a thread a pair and the output a thread a neuron: the pair (or neuron) is the
+    // fastest index, so that a warp's weights are side by side
+    float2 k3t[kK3W * kK3H][kM3 / 2];  // L3 maps (2i, 2i+1) read neighbour sum i: [tap][i]
     float2 a3p[kM3 / 2][4];
-    float2 hwp[kHL / 2][kM3];       // hidden neurons (2q, 2q+1) over every L3 value
+    float2 hwt[kM3][kHL / 2];       // hidden neurons (2q, 2q+1) over every L3 value: [value][q]
     float2 hbp[kHL / 2];            // their biases
     float2 hbnwp[kHL / 2], hbnbp[kHL / 2];
     float htw;                      // tanh slope (one group)
-    float ow[kOut][kHL];
+    float owt[kHL][16];             // [hidden neuron][output]
     float ob[kOut];
     float otw, af;
     float2 negzero;

@@ -14,6 +14,9 @@
 //   a fully connected hidden layer of 384 neurons and 13 outputs (cnn_simd_cntk.cpp:640-963).
 // Map pairs (2i, 2i+1) read the same input and neurons (2q, 2q+1) the same L3 values: each
 // pair runs as packed f32x2 operations, every value keeping the reference's roundings.
+// Bound by latency (one network a SM, its last three layers chains of 110, 96 and 384 terms): 35 us for a 1280x720
+// frame's faces on B200; 52 with 256 threads, the last layers' weights read a row a lane (a cache line each) and
+// the output's products inside its chain.
 #include "kernels.h"
 #include "resample.cuh"
 #include "window_common.cuh"
@@ -23,7 +26,7 @@ namespace ccnn {
 namespace {
 
 using LN = LandmarkNet;
-constexpr int kFT = 256;
+constexpr int kFT = 512;
 constexpr int kC1W = LN::kInW - 3, kC1H = LN::kInH - 3;  // 46 x 48 conv positions
 constexpr int kQ1W = kC1W / 2, kQ1H = kC1H / 2;          // 23 x 24 pooled
 constexpr int kC2W = kQ1W - 2, kC2H = kQ1H - 2;          // 21 x 22
@@ -38,6 +41,7 @@ struct FacialSmem {
             float p2[LN::kM2][kQ2H][kQ2W];
             float s2[LN::kM2][kQ2H][kQ2W];
         } b;
+        float prod[LN::kHL][16];
     } u;
     float a3[LN::kM3];
     float hid[LN::kHL];
@@ -118,10 +122,11 @@ __device__ void landmark_net(const LN& W, FacialSmem& S) {
     if (threadIdx.x < LN::kM3 / 2) {
         const int i = threadIdx.x;
         f2_t acc = 0ull;  // (+0, +0)
+#pragma unroll
         for (int r = 0; r < LN::kK3H; ++r)
 #pragma unroll
             for (int c = 0; c < LN::kK3W; ++c)
-                acc = f2_add(acc, f2_mul(f2_dup(S.u.b.s2[i][r][c]), f2_ld(W.k3p[i][r * LN::kK3W + c]), nz));
+                acc = f2_add(acc, f2_mul(f2_dup(S.u.b.s2[i][r][c]), f2_ld(W.k3t[r * LN::kK3W + c][i]), nz));
         const f2_t av = lrelu_bn2(acc, W.a3p[i], nz);
         S.a3[2 * i] = f2_lo(av);
         S.a3[2 * i + 1] = f2_hi(av);
@@ -131,7 +136,8 @@ __device__ void landmark_net(const LN& W, FacialSmem& S) {
     if (threadIdx.x < LN::kHL / 2) {
         const int q = threadIdx.x;
         f2_t s = f2_ld(W.hbp[q]);
-        for (int j = 0; j < LN::kM3; ++j) s = f2_add(s, f2_mul(f2_dup(S.a3[j]), f2_ld(W.hwp[q][j]), nz));
+#pragma unroll 48
+        for (int j = 0; j < LN::kM3; ++j) s = f2_add(s, f2_mul(f2_dup(S.a3[j]), f2_ld(W.hwt[j][q]), nz));
         s = f2_mul(s, f2_dup(W.htw), nz);
         const f2_t half = f2_pack(0.5f, 0.5f);
         const f2_t v = f2_add(f2_mul(half, tanh_rational2(s, nz), nz), half);
@@ -140,11 +146,15 @@ __device__ void landmark_net(const LN& W, FacialSmem& S) {
         S.hid[2 * q + 1] = f2_hi(h);
     }
     __syncthreads();
-    // outputs (mulC / mulC1_add in neuron order, then tanhW, :885-900, :673-690)
+    // outputs (mulC / mulC1_add in neuron order, then tanhW, :885-900, :673-690): the products by the block, then a
+    // thread an output adds them up
+    for (int it = threadIdx.x; it < LN::kHL * 16; it += kFT) S.u.prod[it / 16][it % 16] = fmul(S.hid[it / 16], W.owt[it / 16][it % 16]);
+    __syncthreads();
     if (threadIdx.x < LN::kOut) {
         const int k = threadIdx.x;
-        float acc = fmul(S.hid[0], W.ow[k][0]);
-        for (int t = 1; t < LN::kHL; ++t) acc = fadd(fmul(S.hid[t], W.ow[k][t]), acc);
+        float acc = S.u.prod[0][k];
+#pragma unroll 16
+        for (int t = 1; t < LN::kHL; ++t) acc = fadd(S.u.prod[t][k], acc);
         float c = fmul(fadd(acc, W.ob[k]), W.otw);
         c = tanh_rational(c);
         S.res[k] = (W.af == 0.f) ? fadd(fmul(0.5f, c), 0.5f) : fmul(W.af, c);

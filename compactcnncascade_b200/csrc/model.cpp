@@ -234,12 +234,12 @@ bool pack_landmarks(const RawModel& m, LandmarkNet* o, std::string* err) {
         act_pair(1, i, o->a2p[i]);
     }
     for (int i = 0; i < LN::kM3 / 2; ++i) {
-        for (int k = 0; k < LN::kK3W * LN::kK3H; ++k) o->k3p[i][k] = make_float2(tap(2, 2 * i, k), tap(2, 2 * i + 1, k));
+        for (int k = 0; k < LN::kK3W * LN::kK3H; ++k) o->k3t[k][i] = make_float2(tap(2, 2 * i, k), tap(2, 2 * i + 1, k));
         act_pair(2, i, o->a3p[i]);
     }
     for (int q = 0; q < LN::kHL / 2; ++q) {
         for (int j = 0; j < LN::kM3; ++j)
-            o->hwp[q][j] = make_float2(m.hw[(size_t)(2 * q) * LN::kM3 + j], m.hw[(size_t)(2 * q + 1) * LN::kM3 + j]);
+            o->hwt[j][q] = make_float2(m.hw[(size_t)(2 * q) * LN::kM3 + j], m.hw[(size_t)(2 * q + 1) * LN::kM3 + j]);
         o->hbp[q] = make_float2(m.hb[2 * q], m.hb[2 * q + 1]);
         o->hbnwp[q] = make_float2(m.hbn[2 * (2 * q)], m.hbn[2 * (2 * q + 1)]);
         o->hbnbp[q] = make_float2(m.hbn[2 * (2 * q) + 1], m.hbn[2 * (2 * q + 1) + 1]);
@@ -247,7 +247,7 @@ bool pack_landmarks(const RawModel& m, LandmarkNet* o, std::string* err) {
     o->htw = m.htw[0];
     // one group, so the output sum visits the hidden neurons in order with weight index t
     for (int k = 0; k < LN::kOut; ++k) {
-        for (int t = 0; t < LN::kHL; ++t) o->ow[k][t] = m.ow[(size_t)k * m.hl + t];
+        for (int t = 0; t < LN::kHL; ++t) o->owt[t][k] = m.ow[(size_t)k * m.hl + t];
         o->ob[k] = m.ob[k];
     }
     o->otw = m.otw;
