@@ -14,15 +14,20 @@
 //   Merger(0.2, del) (:2753-2772), optional rescale for shrunken gray input (:2785-2806).
 //
 // The scan test of a level against the detections of earlier levels has no order dependence,
-// so all 32 warps run it in parallel (one warp per candidate, 32 earlier boxes per ballot).
+// so all warps run it in parallel (one warp per candidate, 32 earlier boxes per ballot).
 // Every box a level appends has the geometry of one of that level's candidates, so the tests
 // against boxes appended during the level (its own scan, then the survivors' pass) are candidate
 // pairs: all warps evaluate them into bit matrices first, and warp 0 then replays the order-
 // dependent decisions with one ballot over the bit words per candidate. Levels with more than
 // kBitMax candidates take the direct route (warp 0 tests the appended boxes 32 at a time). The sort
 // permutes (scale, index) keys. The first clustering pass runs per group of boxes that cannot
-// interact (a warp a group), the second on bit matrices of its pair tests; lists too long for the
-// shared scratch take one warp through the reference's loop.
+// interact (a warp a group, its boxes in the lanes), the second on bit matrices of its pair tests; lists too long
+// for the shared scratch take one warp through the reference's loop. Without drop_detect no candidate depends on
+// another, and the accepted ones are listed at once.
+// Bound by the latency of its dependent steps (one block). On B200, SM cycles of a warm run, before and after the
+// merges took their boxes into lanes, pair tests lost their divisions and doubles, scores were left to a pass after
+// the loop, and the block went from 1,024 to 512 threads: a 1920x1080 frame (221 candidates, 67 boxes) 115 K -> 102 K,
+// a 640x480 one 57 K -> 46 K, a 1280x720 one with facial analysis (83 candidates, no drop_detect) 101 K -> 42 K.
 #include <climits>
 #include <vector>
 
@@ -32,16 +37,21 @@
 
 namespace ccnn {
 
-constexpr int kRT = 1024;
+// most steps are short dependent chains that every warp walks through: 1,024 threads took 2-9 % longer
+constexpr int kRT = 512;
 
-// the candidate's stage-1 pattern rectangle (new_rect, cnn_detector_v3.cpp:1497-1501); the pattern is
-// the stage-1 network's smallest input
-__device__ __forceinline__ Det cand_rect(const Candidate& c, float inv_scale, float scale, int pat_w, int pat_h) {
-    return make_det((int)((float)c.px * inv_scale), (int)((float)c.py * inv_scale), (int)((float)pat_w * inv_scale),
-                    (int)((float)pat_h * inv_scale), 0.f, scale, 0);
-}
-
+// v = (a, a2, b, b2), the two boxes' edges on an axis, in ascending order. Edges of overlapping boxes that are not
+// inside out take one min / max step.
 __device__ __forceinline__ void sort4(int* v) {
+    const int m1 = imax(v[0], v[2]), m2 = imin(v[1], v[3]);
+    if (v[0] <= v[1] && v[2] <= v[3] && m1 <= m2) {
+        const int lo = imin(v[0], v[2]), hi = imax(v[1], v[3]);
+        v[0] = lo;
+        v[1] = m1;
+        v[2] = m2;
+        v[3] = hi;
+        return;
+    }
     // any correct sort gives the same ascending values
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -62,19 +72,6 @@ struct MergeTest {
     int X[4], Y[4];
 };
 
-// fl(a / b) > t for a >= 0, b > 0 and t > 0 (normal floats), without the division: the rounded
-// quotient exceeds t exactly when the real one lies above the midpoint between t and the next float,
-// or on it when the tie rounds to that next float (t's last significand bit is 1). mid * b carries at
-// most 25 + 24 significant bits, so the double product and comparison are exact.
-__device__ __forceinline__ bool quot_gt(float a, float b, float t) {
-    const double mid = 0.5 * ((double)t + (double)nextafterf(t, __int_as_float(0x7f800000)));
-    const double prod = mid * (double)b;
-    const double aa = (double)a;
-    if (aa > prod) return true;
-    if (aa < prod) return false;
-    return (__float_as_uint(t) & 1u) != 0u;
-}
-
 __device__ __forceinline__ MergeTest merge_test(const Det& a, const Det& b, float threshold) {
     MergeTest t;
     t.hit = false;
@@ -82,30 +79,35 @@ __device__ __forceinline__ MergeTest merge_test(const Det& a, const Det& b, floa
     int X[4] = {a.x, a.x2, b.x, b.x2};
     int Y[4] = {a.y, a.y2, b.y, b.y2};
     if (X[0] >= X[3] || X[1] <= X[2] || Y[0] >= Y[3] || Y[1] <= Y[2]) return t;
-    const float S1 = (float)((X[1] - X[0]) * (Y[1] - Y[0]));
-    const float S2 = (float)((X[3] - X[2]) * (Y[3] - Y[2]));
+    const int s1 = (X[1] - X[0]) * (Y[1] - Y[0]);
+    const int s2 = (X[3] - X[2]) * (Y[3] - Y[2]);
     sort4(X);
     sort4(Y);
-    const float su = (float)((X[3] - X[0]) * (Y[3] - Y[0]));
-    const float si = (float)((X[2] - X[1]) * (Y[2] - Y[1]));
+    const int sui = (X[3] - X[0]) * (Y[3] - Y[0]);
+    const int sii = (X[2] - X[1]) * (Y[2] - Y[1]);
     const int CX1 = X[0] + ((X[3] - X[0]) >> 1);
     const int CY1 = Y[0] + ((Y[3] - Y[0]) >> 1);
     const int CX2 = X[1] + ((X[2] - X[1]) >> 1);
     const int CY2 = Y[1] + ((Y[2] - Y[1]) >> 1);
     const int thrC = imin(X[3] - X[0], X[2] - X[1]) >> 1;
     const bool centred = abs(CX1 - CX2) < thrC && abs(CY1 - CY2) < thrC;
-    if (S1 > 0.f && S2 > 0.f && su > 0.f && si >= 0.f && threshold > 0.f) {
-        // r1 = si / S1, r2 = si / S2, r3 = si / su as the reference rounds them, compared without
-        // dividing: min(r1, r2) > threshold is both > threshold, max(r1, r2) > 0.7 is either
-        const bool over = centred && quot_gt(si, su, fmul(0.75f, threshold)) && (quot_gt(si, S1, 0.7f) || quot_gt(si, S2, 0.7f));
-        t.hit = over ? (1.f > threshold) : (quot_gt(si, S1, threshold) && quot_gt(si, S2, threshold));
+    // r1 = si / S1, r2 = si / S2, r3 = si / su as the reference rounds them, compared without dividing:
+    // min(r1, r2) > threshold is both > threshold, max(r1, r2) > 0.7 is either
+    if (s1 > 0 && s1 < kQuotMax && s2 > 0 && s2 < kQuotMax && sui > 0 && sui < kQuotMax && sii >= 0 && sii < kQuotMax && threshold >= 0x1p-12f &&
+        threshold <= 1.f) {
+        const QuotBound bt = quot_bound(__float_as_uint(threshold)), b7 = quot_bound(0x3f333333u);  // 0.7f
+        const bool over = centred && quot_gt_int(sii, sui, quot_bound(__float_as_uint(fmul(0.75f, threshold)))) &&
+                          (quot_gt_int(sii, s1, b7) || quot_gt_int(sii, s2, b7));
+        t.hit = over ? (1.f > threshold) : (quot_gt_int(sii, s1, bt) && quot_gt_int(sii, s2, bt));
+        t.s1_gt_s2 = s1 > s2;
     } else {
+        const float S1 = (float)s1, S2 = (float)s2, su = (float)sui, si = (float)sii;
         const float r1 = fdiv(si, S1), r2 = fdiv(si, S2), r3 = fdiv(si, su);
         float ratio = r1 > r2 ? r2 : r1;
         if (r3 > fmul(0.75f, threshold) && (r1 < r2 ? r2 : r1) > 0.7f && centred) ratio = 1.f;
         t.hit = ratio > threshold;
+        t.s1_gt_s2 = S1 > S2;
     }
-    t.s1_gt_s2 = S1 > S2;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         t.X[i] = X[i];
@@ -300,6 +302,84 @@ __device__ void merge_group_warp(const Det* in, int n, const int* parent, int r,
     }
 }
 
+// The same for a group of at most 32 boxes, lane k its k-th (idx: its index, -1 past the last): the boxes stay in
+// registers, and a test of the running cluster covers all that are left (the boxes of a group are spread over
+// the list, so merge_group_warp takes several tests for the same). The steps are one dependent chain, so where
+// no box is inside out and the whole group's box is below 2^24 pixels the test is cut down to what depends on the
+// growing cluster (`quick`).
+__device__ void merge_group_lanes(const Det* in, int idx, Det* seed_box, int* seed_of) {
+    const int lane = threadIdx.x & 31;
+    constexpr unsigned kAll = 0xffffffffu;
+    unsigned alive = __ballot_sync(kAll, idx >= 0);
+    const Det e = in[imax(idx, 0)];  // a lane past the last repeats a box of the list
+    const int gx0 = __reduce_min_sync(kAll, idx >= 0 ? e.x : INT_MAX), gx1 = __reduce_max_sync(kAll, idx >= 0 ? e.x2 : INT_MIN);
+    const int gy0 = __reduce_min_sync(kAll, idx >= 0 ? e.y : INT_MAX), gy1 = __reduce_max_sync(kAll, idx >= 0 ? e.y2 : INT_MIN);
+    const bool quick = __all_sync(kAll, idx < 0 || (e.x < e.x2 && e.y < e.y2)) && (long long)gx1 - gx0 < kQuotMax && (long long)gy1 - gy0 < kQuotMax &&
+                       ((long long)gx1 - gx0) * ((long long)gy1 - gy0) < kQuotMax;
+    constexpr QuotBound b5 = quot_bound(0x3f000000u), b375 = quot_bound(0x3ec00000u), b7 = quot_bound(0x3f333333u);  // 0.5, 0.75 * 0.5, 0.7
+    const int s2 = quick ? (e.x2 - e.x) * (e.y2 - e.y) : 0;
+    while (alive) {
+        const int s = __ffs(alive) - 1;
+        const int i1 = __shfl_sync(kAll, idx, s);
+        Det nmax = in[i1], nmin = nmax;
+        alive &= alive - 1;
+        unsigned later = alive;  // those not yet passed by this cluster
+        while (later) {
+            bool hit;
+            if (quick) {
+                // merge_test of two boxes with edges in order
+                const int x1 = imax(nmax.x, e.x), x2 = imin(nmax.x2, e.x2), x0 = imin(nmax.x, e.x), x3 = imax(nmax.x2, e.x2);
+                const int y1 = imax(nmax.y, e.y), y2 = imin(nmax.y2, e.y2), y0 = imin(nmax.y, e.y), y3 = imax(nmax.y2, e.y2);
+                const int s1 = (nmax.x2 - nmax.x) * (nmax.y2 - nmax.y);
+                const int su = (x3 - x0) * (y3 - y0), si = (x2 - x1) * (y2 - y1);
+                const int thr_c = imin(x3 - x0, x2 - x1) >> 1;
+                const bool centred = abs((x0 + ((x3 - x0) >> 1)) - (x1 + ((x2 - x1) >> 1))) < thr_c &&
+                                     abs((y0 + ((y3 - y0) >> 1)) - (y1 + ((y2 - y1) >> 1))) < thr_c;
+                const bool over = centred & quot_gt_int(si, su, b375) & (quot_gt_int(si, s1, b7) | quot_gt_int(si, s2, b7));
+                hit = (x1 < x2) & (y1 < y2) & (over | (quot_gt_int(si, s1, b5) & quot_gt_int(si, s2, b5)));
+            } else {
+                hit = merge_test(nmax, e, 0.5f).hit;
+            }
+            const unsigned m = __ballot_sync(kAll, hit) & later;
+            if (!m) break;
+            const int f = __ffs(m) - 1;
+            const int jf = __shfl_sync(kAll, idx, f);
+            const Det ef = in[jf];
+            int X[4] = {nmax.x, nmax.x2, ef.x, ef.x2};
+            int Y[4] = {nmax.y, nmax.y2, ef.y, ef.y2};
+            sort4(X);
+            sort4(Y);
+            nmax.x = imin(nmax.x, X[0]);
+            nmax.y = imin(nmax.y, Y[0]);
+            nmax.x2 = imax(nmax.x2, X[3]);
+            nmax.y2 = imax(nmax.y2, Y[3]);
+            nmin.x = imax(nmin.x, X[1]);
+            nmin.y = imax(nmin.y, Y[1]);
+            nmin.x2 = imin(nmin.x2, X[2]);
+            nmin.y2 = imin(nmin.y2, Y[2]);
+            nmax.score = (nmax.score < ef.score) ? ef.score : nmax.score;
+            nmax.knn = imax(nmax.knn, ef.knn);
+            nmax.scale = (nmax.scale > ef.scale) ? ef.scale : nmax.scale;
+            nmax.num_detect++;
+            if (lane == f) seed_of[jf] = i1;
+            alive &= ~(1u << f);
+            later &= ~((2u << f) - 1u);
+        }
+        Det rr = nmax;
+        rr.x = (nmin.x + nmax.x) >> 1;
+        rr.y = (nmin.y + nmax.y) >> 1;
+        rr.x2 = (nmin.x2 + nmax.x2) >> 1;
+        rr.y2 = (nmin.y2 + nmax.y2) >> 1;
+        rr.w = rr.x2 - rr.x;
+        rr.h = rr.y2 - rr.y;
+        if (lane == 0) {
+            seed_of[i1] = i1;
+            seed_box[i1] = rr;
+        }
+    }
+    __syncwarp();
+}
+
 // Merger(0.5, false) of n <= kGroupMax sorted boxes by the whole block; returns the cluster count
 // (every thread). out: the clusters in reference order; seed_box: n Det of scratch; clus (optional):
 // cluster of every box; ws_a / ws_b: 4n / 3n ints of shared memory.
@@ -314,13 +394,16 @@ __device__ int first_merge_groups(const Det* in, int n, uint8_t* checked, Det* o
     int* seed_of = ws_b + n;
     int* rank_of = ws_b + 2 * n;
     __shared__ int s_groups;
-    for (int j = tid; j < n; j += blockDim.x) {
+    __shared__ uint16_t s_member[kRT / 32][32];
+    const bool one = n <= 32;  // a single warp's worth: no groups
+    if (one && warp == 0) merge_group_lanes(in, lane < n ? lane : -1, seed_box, seed_of);
+    for (int j = tid; j < n && !one; j += blockDim.x) {
         parent[j] = j;
         checked[j] = 0;
     }
     __syncthreads();
     // boxes that overlap or touch share a group
-    for (int i = warp; i < n; i += nwarps) {
+    for (int i = warp; i < n && !one; i += nwarps) {
         const Det bi = in[i];
         const int ax0 = imin(bi.x, bi.x2), ax1 = imax(bi.x, bi.x2), ay0 = imin(bi.y, bi.y2), ay1 = imax(bi.y, bi.y2);
         for (int j = i + 1 + lane; j < n; j += 32) {
@@ -331,7 +414,7 @@ __device__ int first_merge_groups(const Det* in, int n, uint8_t* checked, Det* o
     }
     __syncthreads();
     // groups whose bounding boxes overlap or touch are joined until none do
-    for (;;) {
+    while (!one) {
         for (int j = tid; j < n; j += blockDim.x) {
             int v = parent[j];
             while (v != parent[v]) v = parent[v];
@@ -361,13 +444,27 @@ __device__ int first_merge_groups(const Det* in, int n, uint8_t* checked, Det* o
     // a pass without links left every parent a root: group g = the root; warp w takes the groups
     // w, w + nwarps, ... in order of their roots
     int ord = 0;
-    for (int cb = 0; cb < n; cb += 32) {
+    for (int cb = 0; cb < n && !one; cb += 32) {
         const int j = cb + lane;
         unsigned rm = __ballot_sync(0xffffffffu, j < n && parent[j] == j);
         while (rm) {
             const int g = cb + __ffs(rm) - 1;
             rm &= rm - 1;
-            if (ord++ % nwarps == warp) merge_group_warp(in, n, const_cast<const int*>(ws_a), g, checked, seed_box, seed_of);
+            if (ord++ % nwarps != warp) continue;
+            int members = 0;
+            for (int mb = g & ~31; mb < n; mb += 32) {
+                const int k = mb + lane;
+                const bool in_g = k < n && parent[k] == g;
+                const unsigned mm = __ballot_sync(0xffffffffu, in_g);
+                const int pos = members + __popc(mm & ((1u << lane) - 1u));
+                if (in_g && pos < 32) s_member[warp][pos] = (uint16_t)k;
+                members += __popc(mm);
+            }
+            __syncwarp();
+            if (members <= 32)
+                merge_group_lanes(in, lane < members ? s_member[warp][lane] : -1, seed_box, seed_of);
+            else
+                merge_group_warp(in, n, const_cast<const int*>(ws_a), g, checked, seed_box, seed_of);
         }
     }
     __syncthreads();
@@ -457,12 +554,16 @@ __device__ int second_merge_bits(const Det* in, int n, Det* out, int* src, uint3
 }
 
 constexpr int kMaxLevels = 1024;
-
+// what the loop needs of a level: its scale and its candidates' pattern size
+struct LevelRect {
+    float scale, inv_scale;
+    int w, h;
+};
+constexpr int kLevelSmem = 128;  // levels kept in shared memory (deeper pyramids make the rest from global)
 
 constexpr int kBitMax = 256;              // candidates per level handled with bit matrices
 constexpr int kBitWords = kBitMax / 32;
-constexpr int kOwnVerdict = -kBitMax - 1;  // the candidate's own stage-2/3 verdict
-constexpr int kOwnScore = -kBitMax - 2;    // the candidate's stage-1 score (detection disabled)
+constexpr int kOwnVerdict = -kBitMax - 1;  // the candidate's own stage-2/3 verdict (or stage-1 score, detection disabled)
 
 __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -473,6 +574,7 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
     __shared__ int s_didx[kBitMax];  // D index of the box a candidate appended, or -1
     __shared__ int s_src[kBitMax];   // where that box's score/knn come from
     __shared__ uint32_t s_S[kBitWords], s_T[kBitWords];  // candidate sets of the level (see below)
+    __shared__ LevelRect s_lv[kLevelSmem];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const CascadeConfig& C = a.cfg;
     const int n = *a.n_cand;
@@ -520,14 +622,32 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
     uint32_t* P1 = pre_rows ? reinterpret_cast<uint32_t*>(sm + ((121LL * n + 15) & ~15LL)) : nullptr;
     uint32_t* P2 = pre_rows ? P1 + (size_t)kBitWords * n : nullptr;
     for (int l = tid; l <= nl; l += kRT) s_lvl_start[l] = 0;
+    auto load_level = [&](int l) {
+        const float inv = a.levels[l].inv_scale;
+        return LevelRect{a.levels[l].scale, inv, (int)((float)C.pat_w * inv), (int)((float)C.pat_h * inv)};
+    };
+    for (int l = tid; l < nl && l < kLevelSmem; l += kRT) s_lv[l] = load_level(l);
+    auto level_rect = [&](int l) { return l < kLevelSmem ? s_lv[l] : load_level(l); };
+    // the candidate's stage-1 pattern rectangle (new_rect, cnn_detector_v3.cpp:1497-1501); the pattern is the stage-1
+    // network's smallest input. In the shared copy px and py are made the rectangle's corner below.
+    auto cand_rect = [&](const Candidate& c, const LevelRect& L) {
+        return make_det(fits ? c.px : (int)((float)c.px * L.inv_scale), fits ? c.py : (int)((float)c.py * L.inv_scale), L.w, L.h, 0.f, L.scale, 0);
+    };
     __syncthreads();
     // verdicts and per-level candidate counts (candidates are grouped by level, smallest first)
     for (int i = tid; i < n; i += kRT) {
         const Candidate cd = cands[i];
         if (C.detect_enabled) {
-            const CandResult r = verdict(a.win + (size_t)i * 4, cd, a.levels[cd.level].scale, C);
-            res[i] = r;
+            const CandResult r = verdict(a.win + (size_t)i * 4, cd, level_rect(cd.level).scale, C);
             if (fits) a.results[i] = r;  // kept for inspection
+            res[i] = r;
+            // facial analysis drops a window whose landmarks collapse (cnn_detector_v3.cpp:1750)
+            res[i].pad = r.accepted && !(a.attr && a.attr[i].x);
+        }
+        if (fits) {
+            const float inv = level_rect(cd.level).inv_scale;
+            cands[i].px = (int)((float)cd.px * inv);
+            cands[i].py = (int)((float)cd.py * inv);
         }
         atomicAdd(&s_lvl_start[nl - 1 - cd.level + 1], 1);
     }
@@ -544,13 +664,13 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
             const int k = nl - 1 - cd.level;
             const int g = s_lvl_start[k], m = s_lvl_start[k + 1] - g, i = c - g;
             if (m > kBitMax) continue;
-            const LevelDesc& Lc = a.levels[cd.level];
-            const Det nr = cand_rect(cd, Lc.inv_scale, Lc.scale, C.pat_w, C.pat_h);
+            const LevelRect L = level_rect(cd.level);
+            const Det nr = cand_rect(cd, L);
             const Det ex = rect_shrink(nr, 0.7f);
             for (int w = 0; w < ((i + 31) >> 5); ++w) {
                 const int j = 32 * w + lane;
                 int t = 0;
-                if (j < i) t = drop_test(nr, ex, cand_rect(cands[g + j], Lc.inv_scale, Lc.scale, C.pat_w, C.pat_h));
+                if (j < i) t = drop_test(nr, ex, cand_rect(cands[g + j], L));
                 const uint32_t b1 = __ballot_sync(0xffffffffu, t == 1), b2 = __ballot_sync(0xffffffffu, t == 2);
                 if (lane == 0) {
                     P1[(size_t)c * kBitWords + w] = b1;
@@ -567,322 +687,319 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
     }
 
     int nD = 0;
-    for (int k = 0; k < nl; ++k) {
+    if (!C.drop_detect) {
+        // no candidate depends on another: the accepted ones in order
+        for (int base = 0; base < n; base += kRT) {
+            const int i = base + tid;
+            const bool in = i < n && (!C.detect_enabled || res[i].pad);
+            const uint32_t word = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) s_didx[warp] = __popc(word);
+            __syncthreads();
+            int dst = nD + __popc(word & ((1u << lane) - 1u));
+            for (int w = 0; w < kRT / 32; ++w) {
+                if (w < warp) dst += s_didx[w];
+                nD += s_didx[w];
+            }
+            if (in) {
+                const LevelRect L = level_rect(cands[i].level);
+                const Det nr = cand_rect(cands[i], L);
+                D[dst] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, L.scale, -1 - i);
+            }
+            __syncthreads();
+        }
+    }
+    for (int k = 0; k < nl && C.drop_detect; ++k) {
         const int g = s_lvl_start[k], e = s_lvl_start[k + 1];
         if (g == e) continue;
         const int lev = nl - 1 - k;
-        const LevelDesc& L = a.levels[lev];
-        const float scale = L.scale, inv_scale = L.inv_scale;
+        const LevelRect L = level_rect(lev);
+        const float scale = L.scale;
         const int n_prefix = nD;
 
-        if (C.drop_detect) {
-            // scan test against the detections of earlier levels, one warp per candidate
-            for (int c = g + warp; c < e; c += kRT / 32) {
-                const Det nr = cand_rect(cands[c], inv_scale, scale, C.pat_w, C.pat_h);
-                const Det ex = rect_shrink(nr, 0.7f);
-                int code = -1;
-                for (int base = 0; base < n_prefix; base += 32) {
-                    const int kk = base + lane;
-                    const int t = kk < n_prefix ? drop_test(nr, ex, D[kk]) : 0;
-                    const unsigned m = __ballot_sync(0xffffffffu, t != 0);
-                    if (m) {
-                        const int f = __ffs(m) - 1;
-                        const int tf = __shfl_sync(0xffffffffu, t, f);
-                        code = (base + f) * 2 + (tf - 1);
-                        break;
-                    }
+        // scan test against the detections of earlier levels, one warp per candidate
+        for (int c = g + warp; c < e; c += kRT / 32) {
+            const Det nr = cand_rect(cands[c], L);
+            const Det ex = rect_shrink(nr, 0.7f);
+            int code = -1;
+            for (int base = 0; base < n_prefix; base += 32) {
+                const int kk = base + lane;
+                const int t = kk < n_prefix ? drop_test(nr, ex, D[kk]) : 0;
+                const unsigned m = __ballot_sync(0xffffffffu, t != 0);
+                if (m) {
+                    const int f = __ffs(m) - 1;
+                    const int tf = __shfl_sync(0xffffffffu, t, f);
+                    code = (base + f) * 2 + (tf - 1);
+                    break;
                 }
-                if (lane == 0) first_dec[c] = code;
             }
-            const int m = e - g;
-            const int W = (m + 31) >> 5;
-            // box of candidate i of the level: its rect, score/knn from the end of its copy chain;
-            // facial data travels with a candidate's own accepted box, not with copies
-            auto emit_box = [&](int i) {
-                int r = i, src = s_src[i];
-                while (src < 0 && src > kOwnVerdict) {  // a box of this level: follow it
-                    r = -1 - src;
-                    src = s_src[r];
-                }
-                float sc;
-                int kn;
-                if (src >= 0) {
-                    sc = D[src].score;
-                    kn = D[src].knn;
-                } else if (src == kOwnVerdict) {
-                    sc = res[g + r].score;
-                    kn = res[g + r].knn;
-                } else {
-                    sc = cands[g + r].score;
-                    kn = 0;
-                }
-                const Det nr = cand_rect(cands[g + i], inv_scale, scale, C.pat_w, C.pat_h);
-                D[s_didx[i]] = make_det(nr.x, nr.y, nr.w, nr.h, sc, scale, kn);
-                if (a.fa_scratch) a.fa_scratch[s_didx[i]] = (s_src[i] == kOwnVerdict) ? g + i : -1;
-            };
-            if (pre_rows) {
-                // the level's rows, evaluated before the loop (levels of up to 32 read them in warp 0)
-                if (m > 32 && m <= kBitMax)
-                    for (int it = tid; it < m * W; it += kRT) {
-                        const int i = it / W, w = it - i * W;
-                        s_a1[it] = P1[(size_t)(g + i) * kBitWords + w];
-                        s_a2[it] = P2[(size_t)(g + i) * kBitWords + w];
-                    }
-            } else if (m <= kBitMax) {
-                // candidate-pair tests of this level, one ballot per (row i, word w)
-                for (int it = warp; it < m * W; it += kRT / 32) {
+            if (lane == 0) first_dec[c] = code;
+        }
+        const int m = e - g;
+        const int W = (m + 31) >> 5;
+        // box of candidate i of the level (scores follow after the loop): where its score and knn come from
+        auto emit_box = [&](int i) {
+            const int src = s_src[i];
+            const Det nr = cand_rect(cands[g + i], L);
+            D[s_didx[i]] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, scale, src >= 0 ? src : (src > kOwnVerdict ? s_didx[-1 - src] : -1 - (g + i)));
+        };
+        if (pre_rows) {
+            // the level's rows, evaluated before the loop (levels of up to 32 read them in warp 0)
+            if (m > 32 && m <= kBitMax)
+                for (int it = tid; it < m * W; it += kRT) {
                     const int i = it / W, w = it - i * W;
-                    const int j = 32 * w + lane;
-                    int t = 0;
-                    if (j < i) {
-                        const Det nr = cand_rect(cands[g + i], inv_scale, scale, C.pat_w, C.pat_h);
-                        t = drop_test(nr, rect_shrink(nr, 0.7f), cand_rect(cands[g + j], inv_scale, scale, C.pat_w, C.pat_h));
-                    }
-                    const uint32_t b1 = __ballot_sync(0xffffffffu, t == 1), b2 = __ballot_sync(0xffffffffu, t == 2);
-                    if (lane == 0) {
-                        s_a1[i * W + w] = b1;
-                        s_a2[i * W + w] = b2;
-                    }
+                    s_a1[it] = P1[(size_t)(g + i) * kBitWords + w];
+                    s_a2[it] = P2[(size_t)(g + i) * kBitWords + w];
+                }
+        } else if (m <= kBitMax) {
+            // candidate-pair tests of this level, one ballot per (row i, word w)
+            for (int it = warp; it < m * W; it += kRT / 32) {
+                const int i = it / W, w = it - i * W;
+                const int j = 32 * w + lane;
+                int t = 0;
+                if (j < i) {
+                    const Det nr = cand_rect(cands[g + i], L);
+                    t = drop_test(nr, rect_shrink(nr, 0.7f), cand_rect(cands[g + j], L));
+                }
+                const uint32_t b1 = __ballot_sync(0xffffffffu, t == 1), b2 = __ballot_sync(0xffffffffu, t == 2);
+                if (lane == 0) {
+                    s_a1[i * W + w] = b1;
+                    s_a2[i * W + w] = b2;
                 }
             }
-            __syncthreads();
-            // The order-dependent decisions of the level as fixed points over candidate sets (bit j of
-            // word w = candidate 32w + j). Candidate i's decision depends only on candidates j < i, so
-            // after t rounds the first t candidates are final, and a round that changes nothing has
-            // reached the unique solution, which is the sequential one.
-            //   S: boxes appended during the scan: the first decisive box of candidate i (earlier
-            //      levels first, then S in order) has drop type 1;
-            //   T: boxes appended by the survivors' pass: survivor i overlaps (> 0.5) a box of T
-            //      (a copy), or its stage-2/3 verdict accepts it (or detection is disabled).
-            const bool check = C.detect_enabled != 0;
-            if (m <= 32) {
-                // one word: warp 0 alone, candidate i = lane, its rows and decisions in registers;
-                // a round is one ballot
-                if (warp == 0) {
-                    const int i = lane;
-                    const bool valid = i < m;
-                    int code = -1, acc = 0;
-                    uint32_t r1 = 0u, r2 = 0u;
-                    if (valid) {
-                        code = first_dec[g + i];
-                        acc = C.detect_enabled ? res[g + i].accepted : 1;
-                        if (acc && a.attr && a.attr[g + i].x) acc = 0;  // facial analysis dropped it
-                        r1 = pre_rows ? P1[(size_t)(g + i) * kBitWords] : s_a1[i];
-                        r2 = pre_rows ? P2[(size_t)(g + i) * kBitWords] : s_a2[i];
-                    }
-                    uint32_t S = 0u;
-                    for (int round = 0; round <= m; ++round) {
-                        bool in = false;
-                        if (valid) {
-                            if (code >= 0) {
-                                in = (code & 1) == 0;
-                            } else {
-                                const uint32_t hit = (r1 | r2) & S;
-                                if (hit) in = ((r1 >> (__ffs(hit) - 1)) & 1u) != 0u;
-                            }
-                        }
-                        const uint32_t nS = __ballot_sync(0xffffffffu, in);
-                        if (nS == S) break;
-                        S = nS;
-                    }
-                    // survivors: not decided by the scan
-                    const bool surv_i = valid && code < 0 && ((r1 | r2) & S) == 0u;
-                    uint32_t T = 0u;
-                    for (int round = 0; round <= m; ++round) {
-                        const bool in = surv_i && (acc != 0 || (check && (r1 & T) != 0u));
-                        const uint32_t nT = __ballot_sync(0xffffffffu, in);
-                        if (nT == T) break;
-                        T = nT;
-                    }
-                    // D index (scan appends in candidate order, then the survivors' appends) and the
-                    // source of each box's score/knn
-                    const int nScan = __popc(S);
-                    const uint32_t below = (1u << i) - 1u;
-                    if (valid) {
-                        int dst = -1, src = 0;
-                        if ((S >> i) & 1u) {
-                            dst = nD + __popc(S & below);
-                            src = code >= 0 ? (code >> 1) : -1 - (__ffs((r1 | r2) & S) - 1);
-                        } else if ((T >> i) & 1u) {
-                            dst = nD + nScan + __popc(T & below);
-                            src = C.detect_enabled ? kOwnVerdict : kOwnScore;
-                            if (check && (r1 & T)) src = -1 - (__ffs(r1 & T) - 1);
-                        }
-                        s_didx[i] = dst;
-                        s_src[i] = src;
-                    }
-                    __syncwarp();
-                    if (valid && s_didx[i] >= 0) emit_box(i);
-                    if (lane == 0) s_nD = nD + nScan + __popc(T);
-                }
-                __syncthreads();
-                nD = s_nD;
-                continue;
-            }
-            if (m <= kBitMax) {
-                // several words: a thread a candidate (m <= 256: warps 0..7), block-wide rounds
-                const bool thread_item = tid < m;
-                const int i = tid;
+        }
+        __syncthreads();
+        // The order-dependent decisions of the level as fixed points over candidate sets (bit j of
+        // word w = candidate 32w + j). Candidate i's decision depends only on candidates j < i, so
+        // after t rounds the first t candidates are final, and a round that changes nothing has
+        // reached the unique solution, which is the sequential one.
+        //   S: boxes appended during the scan: the first decisive box of candidate i (earlier
+        //      levels first, then S in order) has drop type 1;
+        //   T: boxes appended by the survivors' pass: survivor i overlaps (> 0.5) a box of T
+        //      (a copy), or its stage-2/3 verdict accepts it (or detection is disabled).
+        const bool check = C.detect_enabled != 0;
+        if (m <= 32) {
+            // one word: warp 0 alone, candidate i = lane, its rows and decisions in registers;
+            // a round is one ballot
+            if (warp == 0) {
+                const int i = lane;
+                const bool valid = i < m;
                 int code = -1, acc = 0;
-                if (thread_item) {
+                uint32_t r1 = 0u, r2 = 0u;
+                if (valid) {
                     code = first_dec[g + i];
-                    acc = C.detect_enabled ? res[g + i].accepted : 1;
-                    if (acc && a.attr && a.attr[g + i].x) acc = 0;  // facial analysis dropped it
+                    acc = C.detect_enabled ? res[g + i].pad : 1;
+                    r1 = pre_rows ? P1[(size_t)(g + i) * kBitWords] : s_a1[i];
+                    r2 = pre_rows ? P2[(size_t)(g + i) * kBitWords] : s_a2[i];
                 }
-                if (tid < kBitWords) {
-                    s_S[tid] = 0u;
-                    s_T[tid] = 0u;
-                }
-                __syncthreads();
-                bool inS = false;
+                uint32_t S = 0u;
                 for (int round = 0; round <= m; ++round) {
                     bool in = false;
-                    if (thread_item) {
+                    if (valid) {
                         if (code >= 0) {
                             in = (code & 1) == 0;
                         } else {
-                            for (int w = 0; w < W; ++w) {
-                                const uint32_t hit = (s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w];
-                                if (hit) {
-                                    in = (s_a1[i * W + w] >> (__ffs(hit) - 1)) & 1u;
-                                    break;
-                                }
-                            }
+                            const uint32_t hit = (r1 | r2) & S;
+                            if (hit) in = ((r1 >> (__ffs(hit) - 1)) & 1u) != 0u;
                         }
                     }
-                    const uint32_t word = __ballot_sync(0xffffffffu, in);
-                    __syncthreads();  // every thread has read the previous round's S
-                    const bool changed = (lane == 0 && warp < W && s_S[warp] != word);
-                    if (lane == 0 && warp < W) s_S[warp] = word;
-                    inS = in;
-                    if (!__syncthreads_or(changed)) break;
+                    const uint32_t nS = __ballot_sync(0xffffffffu, in);
+                    if (nS == S) break;
+                    S = nS;
                 }
                 // survivors: not decided by the scan
-                bool surv_i = false;
-                if (thread_item && code < 0) {
-                    surv_i = true;
-                    for (int w = 0; w < W; ++w)
-                        if ((s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w]) {
-                            surv_i = false;
-                            break;
-                        }
-                }
+                const bool surv_i = valid && code < 0 && ((r1 | r2) & S) == 0u;
+                uint32_t T = 0u;
                 for (int round = 0; round <= m; ++round) {
-                    bool in = false;
-                    if (surv_i) {
-                        in = acc != 0;
-                        if (check)
-                            for (int w = 0; w < W && !in; ++w) in = (s_a1[i * W + w] & s_T[w]) != 0u;
+                    const bool in = surv_i && (acc != 0 || (check && (r1 & T) != 0u));
+                    const uint32_t nT = __ballot_sync(0xffffffffu, in);
+                    if (nT == T) break;
+                    T = nT;
+                }
+                // D index (scan appends in candidate order, then the survivors' appends) and the
+                // source of each box's score/knn
+                const int nScan = __popc(S);
+                const uint32_t below = (1u << i) - 1u;
+                if (valid && (((S | T) >> i) & 1u)) {
+                    // the box of candidate j < i of the level that decided this one
+                    const uint32_t by = (S >> i) & 1u ? (r1 | r2) & S : (check ? r1 & T : 0u);
+                    const uint32_t before = by ? (by & (0u - by)) - 1u : 0u;  // candidates in front of j
+                    int dst, src;
+                    if ((S >> i) & 1u) {
+                        dst = nD + __popc(S & below);
+                        src = code >= 0 ? code >> 1 : nD + __popc(S & before);
+                    } else {
+                        dst = nD + nScan + __popc(T & below);
+                        src = by ? nD + nScan + __popc(T & before) : -1 - (g + i);
                     }
-                    const uint32_t word = __ballot_sync(0xffffffffu, in);
-                    __syncthreads();
-                    const bool changed = (lane == 0 && warp < W && s_T[warp] != word);
-                    if (lane == 0 && warp < W) s_T[warp] = word;
-                    if (!__syncthreads_or(changed)) break;
+                    const Det nr = cand_rect(cands[g + i], L);
+                    D[dst] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, scale, src);
                 }
-                int nScan = 0, nSurv = 0;
-                for (int w = 0; w < W; ++w) {
-                    nScan += __popc(s_S[w]);
-                    nSurv += __popc(s_T[w]);
-                }
-                if (thread_item) {
-                    const uint32_t below = (1u << (i & 31)) - 1u;
-                    int dst = -1, src = 0;
-                    if (inS) {
-                        int r = 0;
-                        for (int w = 0; w < (i >> 5); ++w) r += __popc(s_S[w]);
-                        dst = nD + r + __popc(s_S[i >> 5] & below);
-                        if (code >= 0) {
-                            src = code >> 1;
-                        } else {
-                            for (int w = 0; w < W; ++w) {
-                                const uint32_t hit = (s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w];
-                                if (hit) {
-                                    src = -1 - (32 * w + __ffs(hit) - 1);
-                                    break;
-                                }
-                            }
-                        }
-                    } else if ((s_T[i >> 5] >> (i & 31)) & 1u) {
-                        int r = 0;
-                        for (int w = 0; w < (i >> 5); ++w) r += __popc(s_T[w]);
-                        dst = nD + nScan + r + __popc(s_T[i >> 5] & below);
-                        src = C.detect_enabled ? kOwnVerdict : kOwnScore;
-                        if (check)
-                            for (int w = 0; w < W; ++w) {
-                                const uint32_t hit = s_a1[i * W + w] & s_T[w];
-                                if (hit) {
-                                    src = -1 - (32 * w + __ffs(hit) - 1);
-                                    break;
-                                }
-                            }
-                    }
-                    s_didx[i] = dst;
-                    s_src[i] = src;
-                }
-                __syncthreads();
-                if (thread_item && s_didx[i] >= 0) emit_box(i);
-                nD += nScan + nSurv;
-                __syncthreads();
-                continue;
+                if (lane == 0) s_nD = nD + nScan + __popc(T);
             }
-            if (warp == 0) {
-                int nS = 0;
-                for (int c = g; c < e; ++c) {
-                    const int code = first_dec[c];
-                    int k0 = -1, type = 0;
-                    Det nr;
+            __syncthreads();
+            nD = s_nD;
+            continue;
+        }
+        if (m <= kBitMax) {
+            // several words: a thread a candidate (m <= 256: warps 0..7), block-wide rounds
+            const bool thread_item = tid < m;
+            const int i = tid;
+            int code = -1, acc = 0;
+            if (thread_item) {
+                code = first_dec[g + i];
+                acc = C.detect_enabled ? res[g + i].pad : 1;
+            }
+            if (tid < kBitWords) {
+                s_S[tid] = 0u;
+                s_T[tid] = 0u;
+            }
+            __syncthreads();
+            bool inS = false;
+            for (int round = 0; round <= m; ++round) {
+                bool in = false;
+                if (thread_item) {
                     if (code >= 0) {
-                        k0 = code >> 1;
-                        type = (code & 1) + 1;
-                    } else if (nD > n_prefix) {
-                        nr = cand_rect(cands[c], inv_scale, scale, C.pat_w, C.pat_h);
-                        const Det ex = rect_shrink(nr, 0.7f);
-                        for (int base = n_prefix; base < nD; base += 32) {
-                            const int kk = base + lane;
-                            const int t = kk < nD ? drop_test(nr, ex, D[kk]) : 0;
-                            const unsigned m = __ballot_sync(0xffffffffu, t != 0);
-                            if (m) {
-                                const int f = __ffs(m) - 1;
-                                type = __shfl_sync(0xffffffffu, t, f);
-                                k0 = base + f;
+                        in = (code & 1) == 0;
+                    } else {
+                        for (int w = 0; w < W; ++w) {
+                            const uint32_t hit = (s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w];
+                            if (hit) {
+                                in = (s_a1[i * W + w] >> (__ffs(hit) - 1)) & 1u;
                                 break;
                             }
                         }
                     }
-                    if (k0 >= 0) {
-                        if (type == 1) {
-                            if (lane == 0) {
-                                nr = cand_rect(cands[c], inv_scale, scale, C.pat_w, C.pat_h);
-                                const Det src = D[k0];
-                                D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, src.score, scale, src.knn);
-                                if (a.fa_scratch) a.fa_scratch[nD] = -1;
-                            }
-                            nD++;
-                            __syncwarp();
-                        }
-                        continue;
+                }
+                const uint32_t word = __ballot_sync(0xffffffffu, in);
+                __syncthreads();  // every thread has read the previous round's S
+                const bool changed = (lane == 0 && warp < W && s_S[warp] != word);
+                if (lane == 0 && warp < W) s_S[warp] = word;
+                inS = in;
+                if (!__syncthreads_or(changed)) break;
+            }
+            // survivors: not decided by the scan
+            bool surv_i = false;
+            if (thread_item && code < 0) {
+                surv_i = true;
+                for (int w = 0; w < W; ++w)
+                    if ((s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w]) {
+                        surv_i = false;
+                        break;
                     }
-                    if (lane == 0) surv[nS] = c;
-                    nS++;
+            }
+            for (int round = 0; round <= m; ++round) {
+                bool in = false;
+                if (surv_i) {
+                    in = acc != 0;
+                    if (check)
+                        for (int w = 0; w < W && !in; ++w) in = (s_a1[i * W + w] & s_T[w]) != 0u;
                 }
-                if (lane == 0) {
-                    s_nS = nS;
-                    s_nD = nD;
+                const uint32_t word = __ballot_sync(0xffffffffu, in);
+                __syncthreads();
+                const bool changed = (lane == 0 && warp < W && s_T[warp] != word);
+                if (lane == 0 && warp < W) s_T[warp] = word;
+                if (!__syncthreads_or(changed)) break;
+            }
+            int nScan = 0, nSurv = 0;
+            for (int w = 0; w < W; ++w) {
+                nScan += __popc(s_S[w]);
+                nSurv += __popc(s_T[w]);
+            }
+            if (thread_item) {
+                const uint32_t below = (1u << (i & 31)) - 1u;
+                int dst = -1, src = 0;
+                if (inS) {
+                    int r = 0;
+                    for (int w = 0; w < (i >> 5); ++w) r += __popc(s_S[w]);
+                    dst = nD + r + __popc(s_S[i >> 5] & below);
+                    if (code >= 0) {
+                        src = code >> 1;
+                    } else {
+                        for (int w = 0; w < W; ++w) {
+                            const uint32_t hit = (s_a1[i * W + w] | s_a2[i * W + w]) & s_S[w];
+                            if (hit) {
+                                src = -1 - (32 * w + __ffs(hit) - 1);
+                                break;
+                            }
+                        }
+                    }
+                } else if ((s_T[i >> 5] >> (i & 31)) & 1u) {
+                    int r = 0;
+                    for (int w = 0; w < (i >> 5); ++w) r += __popc(s_T[w]);
+                    dst = nD + nScan + r + __popc(s_T[i >> 5] & below);
+                    src = kOwnVerdict;
+                    if (check)
+                        for (int w = 0; w < W; ++w) {
+                            const uint32_t hit = s_a1[i * W + w] & s_T[w];
+                            if (hit) {
+                                src = -1 - (32 * w + __ffs(hit) - 1);
+                                break;
+                            }
+                        }
                 }
+                s_didx[i] = dst;
+                s_src[i] = src;
             }
             __syncthreads();
-            nD = s_nD;
+            if (thread_item && s_didx[i] >= 0) emit_box(i);
+            nD += nScan + nSurv;
+            __syncthreads();
+            continue;
         }
+        if (warp == 0) {
+            int nS = 0;
+            for (int c = g; c < e; ++c) {
+                const int code = first_dec[c];
+                int k0 = -1, type = 0;
+                Det nr;
+                if (code >= 0) {
+                    k0 = code >> 1;
+                    type = (code & 1) + 1;
+                } else if (nD > n_prefix) {
+                    nr = cand_rect(cands[c], L);
+                    const Det ex = rect_shrink(nr, 0.7f);
+                    for (int base = n_prefix; base < nD; base += 32) {
+                        const int kk = base + lane;
+                        const int t = kk < nD ? drop_test(nr, ex, D[kk]) : 0;
+                        const unsigned m = __ballot_sync(0xffffffffu, t != 0);
+                        if (m) {
+                            const int f = __ffs(m) - 1;
+                            type = __shfl_sync(0xffffffffu, t, f);
+                            k0 = base + f;
+                            break;
+                        }
+                    }
+                }
+                if (k0 >= 0) {
+                    if (type == 1) {
+                        if (lane == 0) {
+                            nr = cand_rect(cands[c], L);
+                            D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, scale, k0);
+                        }
+                        nD++;
+                        __syncwarp();
+                    }
+                    continue;
+                }
+                if (lane == 0) surv[nS] = c;
+                nS++;
+            }
+            if (lane == 0) {
+                s_nS = nS;
+                s_nD = nD;
+            }
+        }
+        __syncthreads();
+        nD = s_nD;
 
         if (warp == 0) {
-            const int nS = C.drop_detect ? s_nS : (e - g);
+            const int nS = s_nS;
             const int rect_size = nD;
             for (int si = 0; si < nS; ++si) {
-                const int c = C.drop_detect ? surv[si] : g + si;
+                const int c = surv[si];
                 const Candidate cd = cands[c];
-                const Det nr = cand_rect(cd, inv_scale, scale, C.pat_w, C.pat_h);
-                if (C.drop_detect && C.detect_enabled && nD > rect_size) {
+                const Det nr = cand_rect(cd, L);
+                if (C.detect_enabled && nD > rect_size) {
                     int k0 = -1;
                     for (int base = rect_size; base < nD; base += 32) {
                         const int kk = base + lane;
@@ -894,32 +1011,15 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
                         }
                     }
                     if (k0 >= 0) {
-                        if (lane == 0) {
-                            const Det src = D[k0];
-                            D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, src.score, scale, src.knn);
-                            if (a.fa_scratch) a.fa_scratch[nD] = -1;
-                        }
+                        if (lane == 0) D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, scale, k0);
                         nD++;
                         __syncwarp();
                         continue;
                     }
                 }
-                if (!C.detect_enabled) {
-                    if (lane == 0) {
-                        D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, cd.score, scale, 0);
-                        if (a.fa_scratch) a.fa_scratch[nD] = -1;
-                    }
+                if (!C.detect_enabled || res[c].pad) {
+                    if (lane == 0) D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, 0.f, scale, -1 - c);
                     nD++;
-                } else {
-                    const CandResult r = res[c];
-                    // facial analysis drops a window whose landmarks collapse (cnn_detector_v3.cpp:1750)
-                    if (r.accepted && !(a.attr && a.attr[c].x)) {
-                        if (lane == 0) {
-                            D[nD] = make_det(nr.x, nr.y, nr.w, nr.h, r.score, scale, r.knn);
-                            if (a.fa_scratch) a.fa_scratch[nD] = c;
-                        }
-                        nD++;
-                    }
                 }
                 __syncwarp();
             }
@@ -929,6 +1029,23 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
         nD = s_nD;
     }
 
+    // scores and knn: a box's knn field holds the box it is a copy of, or -1 - its own candidate, so each copy chain
+    // ends at a candidate (kept in num_detect until every chain has been read). Facial data travels with a
+    // candidate's own accepted box, not with copies.
+    for (int i = tid; i < nD; i += kRT) {
+        int src = D[i].knn;
+        if (a.fa_scratch) a.fa_scratch[i] = src < 0 && C.detect_enabled ? -1 - src : -1;
+        while (src >= 0) src = D[src].knn;
+        D[i].num_detect = -1 - src;
+    }
+    __syncthreads();
+    for (int i = tid; i < nD; i += kRT) {
+        const int c = D[i].num_detect;
+        D[i].score = C.detect_enabled ? res[c].score : cands[c].score;
+        D[i].knn = C.detect_enabled ? res[c].knn : 0;
+        D[i].num_detect = 0;
+    }
+    __syncthreads();  // the keys below take the place of the candidates and verdicts
     // raw list (reference order) to global memory for inspection; the reversed list is sorted by
     // permuting (scale, index) keys (the first region is free once the levels are done)
     if (fits)
@@ -1056,44 +1173,64 @@ __device__ __forceinline__ void replay_body(const ReplayArgs& a) {
         f.num_detect = d.num_detect;
         f.pad = 0;
         f.gender = f.smile = f.glasses = -1;
-        if (a.fa_scratch) {
-            // CompactCNNLibAPI_v2.cpp:296-319: each attribute is the element at size/2 of the
-            // merged box's facial data sorted in descending order
-            const int c = a.fa_scratch[3 * a.face_cap + a.fa_scratch[4 * a.face_cap + i]];
-            const int* rcand = a.fa_scratch + a.face_cap;
-            const int* cl = a.fa_scratch + 2 * a.face_cap;
-            int size = 0;
-            for (int r = 0; r < nD; ++r)
-                if (cl[r] == c && rcand[r] >= 0) size++;
-            if (size > 0) {
-                const int k = size / 2;
-                int outv[3];
-                for (int q = 0; q < 3; ++q) {
-                    // the k-th largest value (0-based): a value v with #(> v) <= k < #(>= v)
-                    outv[q] = -1;
-                    for (int r = 0; r < nD && outv[q] == -1; ++r) {
-                        if (cl[r] != c || rcand[r] < 0) continue;
-                        const int4 at = a.attr[rcand[r]];
-                        const int v = q == 0 ? at.y : (q == 1 ? at.z : at.w);
-                        int gt = 0, ge = 0;
-                        for (int u = 0; u < nD; ++u) {
-                            if (cl[u] != c || rcand[u] < 0) continue;
-                            const int4 bu = a.attr[rcand[u]];
-                            const int w = q == 0 ? bu.y : (q == 1 ? bu.z : bu.w);
-                            gt += w > v;
-                            ge += w >= v;
-                        }
-                        if (gt <= k && k < ge) outv[q] = v;
-                    }
-                }
-                f.gender = outv[0];
-                f.smile = outv[1];
-                f.glasses = outv[2];
-            }
-        }
         a.faces[i] = f;
     }
     if (tid == 0) *a.n_faces = nF;
+    if (a.fa_scratch) {
+        // CompactCNNLibAPI_v2.cpp:296-319: each attribute is the element at size/2 of the merged box's facial
+        // data sorted in descending order: a value v with #(> v) <= k < #(>= v). A warp a (face, attribute), a lane
+        // a raw box, on the clusters and values gathered into shared memory (global where they don't fit).
+        constexpr int kStage = kBitMax * kBitWords / 4;
+        const int* rcand = a.fa_scratch + cap;
+        int* st_cl = reinterpret_cast<int*>(s_a1);
+        const bool staged = nD <= kStage;
+        __syncthreads();  // the scratch's last users are done, and the faces are written
+        auto cluster_of = [&](int r) { return rcand[r] >= 0 ? clus[r] : -1; };
+        auto value_of = [&](int r, int q) {
+            const int4 at = a.attr[rcand[r]];
+            return q == 0 ? at.y : (q == 1 ? at.z : at.w);
+        };
+        for (int r = tid; r < nD && staged; r += kRT) {
+            const int c = cluster_of(r);
+            st_cl[4 * r] = c;
+            for (int q = 0; q < 3; ++q) st_cl[4 * r + 1 + q] = c >= 0 ? value_of(r, q) : 0;
+        }
+        __syncthreads();
+        auto cl = [&](int r) { return staged ? st_cl[4 * r] : cluster_of(r); };
+        auto val = [&](int r, int q) { return staged ? st_cl[4 * r + 1 + q] : value_of(r, q); };
+        for (int it = warp; it < 3 * imin(nF, cap); it += kRT / 32) {
+            const int i = it / 3, q = it - 3 * i;
+            const int c = keepmap[fsrc[i]];
+            int size = 0;
+            for (int r0 = 0; r0 < nD; r0 += 32) size += __popc(__ballot_sync(0xffffffffu, r0 + lane < nD && cl(r0 + lane) == c));
+            const int k = size / 2;
+            int out = -1;
+            for (int r0 = 0; r0 < nD && size > 0; r0 += 32) {
+                const int r = r0 + lane;
+                const bool mine = r < nD && cl(r) == c;
+                if (!__any_sync(0xffffffffu, mine)) continue;
+                const int v = mine ? val(r, q) : 0;
+                int gt = 0, ge = 0;
+                for (int u = 0; u < nD; ++u) {
+                    if (cl(u) != c) continue;
+                    const int w = val(u, q);
+                    gt += w > v;
+                    ge += w >= v;
+                }
+                const unsigned ok = __ballot_sync(0xffffffffu, mine && gt <= k && k < ge);
+                if (ok) {
+                    out = __shfl_sync(0xffffffffu, v, __ffs(ok) - 1);
+                    break;
+                }
+            }
+            if (lane == 0) {
+                FaceOut& f = a.faces[i];
+                if (q == 0) f.gender = out;
+                else if (q == 1) f.smile = out;
+                else f.glasses = out;
+            }
+        }
+    }
     if (a.host_faces) {
         // the result straight into the caller's page-locked memory, a warp's stores side by side (two copies
         // after the kernel took 5 us of a frame's latency)

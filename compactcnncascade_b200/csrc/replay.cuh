@@ -64,12 +64,40 @@ CCNN_HD Det rect_shrink(const Det& r, float s) {
     return make_det(r.x + (sx >> 1), r.y + (sy >> 1), r.w - sx, r.h - sy, 0.f, 0.f, 0);
 }
 
+// fl(a / b) > t for integers 0 <= a < 2^24, 0 < b < 2^24 (exact as floats) and t in [2^-13, 1], without dividing:
+// the rounded quotient exceeds t exactly when the real one lies above the midpoint of t and the next float,
+// or on it when the tie rounds to that next float (t's last significand bit is 1). With t = m 2^-e the midpoint
+// is (2m + 1) 2^-(e + 1), so the comparison is one of 64-bit integers (a division, or the product in double that
+// took its place, was most of a pair test's latency).
+struct QuotBound {
+    uint32_t mid;   // 2m + 1
+    int shift;      // e + 1
+    bool tie_up;
+};
+CCNN_HD constexpr QuotBound quot_bound(uint32_t t_bits) {
+    return QuotBound{2u * ((t_bits & 0x7fffffu) | 0x800000u) + 1u, 151 - (int)(t_bits >> 23), (t_bits & 1u) != 0u};
+}
+CCNN_HD bool quot_gt_int(int a, int b, const QuotBound& q) {
+    const uint64_t lhs = (uint64_t)(uint32_t)a << q.shift, rhs = (uint64_t)q.mid * (uint32_t)b;
+    return lhs > rhs || (lhs == rhs && q.tie_up);
+}
+constexpr int kQuotMax = 1 << 24;
+
 // DropDetection's test of one earlier detection (cnn_detector_v3.cpp:1820-1840):
 // 0 = not decisive, 1 = overlap > 0.5 (a copy is appended, candidate dropped), 2 = dropped
 CCNN_HD int drop_test(const Det& nr, const Det& exp_r, const Det& e) {
-    const float ov = rect_overlap(nr, e);
-    if (ov == 0.f) return 0;
-    if (ov > 0.5f) return 1;
+    if (nr.x > e.x2 || e.x > nr.x2 || nr.y > e.y2 || e.y > nr.y2) return 0;
+    const int X0 = imin(nr.x, e.x), X1 = imax(nr.x, e.x), X2 = imin(nr.x2, e.x2), X3 = imax(nr.x2, e.x2);
+    const int Y0 = imin(nr.y, e.y), Y1 = imax(nr.y, e.y), Y2 = imin(nr.y2, e.y2), Y3 = imax(nr.y2, e.y2);
+    const int su = (X3 - X0) * (Y3 - Y0), si = (X2 - X1) * (Y2 - Y1);
+    if (su > 0 && su < kQuotMax && si >= 0 && si < kQuotMax) {
+        if (si == 0) return 0;
+        if (quot_gt_int(si, su, quot_bound(0x3f000000u))) return 1;  // 0.5f
+    } else {
+        const float ov = (float)si / (float)su;
+        if (ov == 0.f) return 0;
+        if (ov > 0.5f) return 1;
+    }
     if (rect_intersects(e, exp_r) == exp_r.w * exp_r.h) return 2;
     return 0;
 }
