@@ -86,6 +86,7 @@ Detector::~Detector() {
     clear();
     if (order_ev_) cudaEventDestroy(order_ev_);
     if (d_lnet_) cudaFree(d_lnet_);
+    if (d_wn_) cudaFree(d_wn_);
     if (d_lg_) cudaFree(d_lg_);
 }
 
@@ -348,6 +349,8 @@ ccnn_status Detector::init() {
         if (!d_lg_) CCNN_CUDA(cudaMalloc(&d_lg_, 3 * sizeof(LegacyNet)));
         CCNN_CUDA(cudaMemcpy(d_lg_, h_lg_.get(), 3 * sizeof(LegacyNet), cudaMemcpyHostToDevice));
     }
+    if (!d_wn_) CCNN_CUDA(cudaMalloc(&d_wn_, sizeof(WindowNets)));
+    CCNN_CUDA(cudaMemcpy(d_wn_, wn_.get(), sizeof(WindowNets), cudaMemcpyHostToDevice));
     if (h_lnet_) {
         if (!d_lnet_) CCNN_CUDA(cudaMalloc(&d_lnet_, sizeof(LandmarkNet)));
         CCNN_CUDA(cudaMemcpy(d_lnet_, h_lnet_.get(), sizeof(LandmarkNet), cudaMemcpyHostToDevice));
@@ -823,7 +826,7 @@ ccnn_status Detector::enqueue_kernels(Slot& s, const Plan& p) {
     CCNN_CUDA(launch_cand_write(p.d_chunks, (int)p.chunks.size(), p.d_levels, s.d_resp, cfg_.thr1, s.d_counts, s.d_cands, s.d_ncand,
                                 (int)cand_cap_, s.st));
     if (detect_enabled_)
-        CCNN_CUDA(launch_window(*wn_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_,
+        CCNN_CUDA(launch_window(*wn_, d_wn_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_,
                                 window_grid_, s.st, legacy_ ? d_lg_ : nullptr, window_ctas_per_sm_));
     if (s.d_attr)
         CCNN_CUDA(launch_facial(d_lnet_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_, s.d_attr,
@@ -1424,7 +1427,7 @@ ccnn_status Detector::profile(int iters, float* ms, int n_ms) {
                                     (int)cand_cap_, s.st));
         CCNN_CUDA(cudaEventRecord(ev[5], s.st));
         if (detect_enabled_)
-            CCNN_CUDA(launch_window(*wn_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_,
+            CCNN_CUDA(launch_window(*wn_, d_wn_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_,
                                     window_grid_, s.st, legacy_ ? d_lg_ : nullptr, window_ctas_per_sm_));
         if (s.d_attr)
             CCNN_CUDA(launch_facial(d_lnet_, s.d_gray, s.gray_pitch, p.gw, p.gh, s.d_cands, s.d_ncand, p.d_levels, s.d_win, cfg_,
@@ -1676,7 +1679,7 @@ ccnn_status Detector::enqueue_batch_kernels(BatchCtx& c, const Plan& p, int B) {
     int* err = c.d_sync + 1 + kBatchStages * B;
     CCNN_CUDA(launch_stage1_batch(w1_, F, Q, p.d_levels, sync, err, grid, st));
     CCNN_CUDA(launch_cand_write_batch(p.d_chunks, (int)p.chunks.size(), p.d_levels, F, C, B, cfg_.thr1, (int)cand_cap_, st));
-    if (detect_enabled_) CCNN_CUDA(launch_window_batch(*wn_, WB, gpitch, p.gw, p.gh, p.d_levels, cfg_, window_grid_, st, window_ctas_per_sm_));
+    if (detect_enabled_) CCNN_CUDA(launch_window_batch(*wn_, d_wn_, WB, gpitch, p.gw, p.gh, p.d_levels, cfg_, window_grid_, st, window_ctas_per_sm_));
     CCNN_CUDA(launch_replay_batch(c.d_rargs, B, st));
     const long long face_cap = std::max<long long>(cand_cap_, kHostFaces);
     CCNN_CUDA(cudaMemcpyAsync(c.h_nf, c.d_nf, sizeof(int) * B, cudaMemcpyDeviceToHost, st));

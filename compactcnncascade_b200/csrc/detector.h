@@ -192,6 +192,7 @@ class Detector {
     std::string model_paths_[3];
     Stage1W w1_{};
     std::unique_ptr<WindowNets> wn_;
+    WindowNets* d_wn_ = nullptr;     // the window networks in device memory too
     LandmarkNet* d_lnet_ = nullptr;  // facial-analysis network (device memory), when enabled
     std::unique_ptr<LandmarkNet> h_lnet_;  // its host copy
     // legacy model family (format 1.0): the three networks on the host and in device memory

@@ -15,6 +15,12 @@
 // retry, drop_detect) is decided by the replay kernel, so the verdicts are the same while all
 // items run in parallel.
 //
+// Bound by latency and barriers as much as by the fp32 pipe: an item is a chain of small layers. With L1 packed over
+// pixels 11 columns apart (operands load as pairs; map pairs needed every input converted and duplicated), weights
+// loaded once for four positions, the layers whose lanes read different maps taken off the constant bank, and the
+// crop a row a warp, 32 gated 1920x1080 frames on B200 go from 1.64 to 1.50 ms and 16 monochrome 1280x720 ones from
+// 0.88 to 0.79 ms.
+//
 // One CTA (256 threads) per work item, persistent over the item list. The networks run
 // entirely in shared memory: L1 (6 maps, 44x48 -> pooled 22x24), neighbour sums, L2 (12 maps,
 // 20x22 -> pooled 10x11), sums, L3 (24 maps, 7w x 8h -> 4x4), hidden layer and output neuron.
@@ -30,19 +36,34 @@ constexpr int kP1W = 22, kP1H = 24;   // pooled L1 of a 47x51 window
 constexpr int kP2W = 10, kP2H = 11;   // pooled L2
 constexpr int kOutN = 16;             // 4x4 response map
 
+constexpr int kHalfW = kP1W / 2;      // 11: L1 pixels x and x + 11 of a row run as a packed pair
+constexpr int kP1Pairs = kHalfW * kP1H;
+constexpr int kInPairs = 2 * kHalfW + 3;  // 25 columns of a row of input pairs
+
 struct WindowSmem {
     uint8_t crop[kCropH][kCropW + 3];
     int hist[256];
     int lut[256];
     float s1[6][kP1H][kP1W + 1];
-    float p2[12][kP2H][kP2W + 1];
-    float s2[12][kP2H][kP2W + 1];
-    float a3[24][kOutN];
-    float hbuf[84][kOutN];
+    union {
+        // the network's input: column c next to column c + 22 (the windows of L1 pixels x and x + 11 load as packed
+        // pairs), even columns, then odd ones (L1 steps by two); the row stride spreads a warp's rows over the banks
+        float2 in[kCropH][2][15];
+        struct {  // after L1
+            float p2[12][kP2H][kP2W + 1];
+            float s2[12][kP2H][kP2W + 1];
+            float a3[24][kOutN];
+        } l;
+    } u;
+    union {
+        alignas(16) float2 k3[12][56];  // L3 taps of the network that runs
+        float hbuf[84][kOutN];          // after L3
+    } v;
     float out[kOutN];
-    float l1rest[32][6];  // pooled L1 maps of the partial pass's pixels
+    float2 l1rest[32][6];  // pooled L1 maps of the partial pass's pixels
     int geo[4];
 };
+static_assert(kInPairs <= 30, "columns of an input row");
 
 // mode: 0 = stage-2 view (columns 2..48), 1 = mirrored (46 - x), 2 = plain (columns 0..46)
 __device__ __forceinline__ float win_in(const WindowSmem& S, int mode, int x, int y) {
@@ -50,67 +71,86 @@ __device__ __forceinline__ float win_in(const WindowSmem& S, int mode, int x, in
     return (float)S.crop[y][c];
 }
 
+// Two consecutive duplicated parameters by one 16-byte constant load.
+__device__ __forceinline__ ulonglong2 ld_two(const float2* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+// One CNTK window network. W: its parameters as kernel parameters (warp-uniform constant loads); G: the same in
+// global memory, for the layers whose lanes read different maps (their constant loads took a pass a map: L3's 56
+// taps 90 cycles each): L3's taps are copied to shared memory while L1 and L2 run.
 template <class NW>
-__device__ void window_net(const NW& W, WindowSmem& S, int mode) {
-    static_assert(NW::kM1 % 2 == 0 && NW::kM2 % 2 == 0 && NW::kM3 % 2 == 0 && NW::kHS % 2 == 0, "maps and neurons run in pairs");
+__device__ void window_net(const NW& W, const NW* __restrict__ G, WindowSmem& S, int mode) {
+    static_assert(NW::kM1 == 6 && NW::kM2 == 12 && NW::kM3 == 24 && NW::kK3W * NW::kK3H == 56 && NW::kHS % 2 == 0, "shared-memory layout");
     const f2_t nz = f2_ld(W.negzero);
-    // L1: conv 4x4 + folded BN/LReLU + 2x2 max, then neighbour sums (add / add2); every map pair
-    // reads the same window, so it runs as one packed pair. Whole passes of kWT pixels run every map
-    // pair per thread; the pixels of the last, partial pass are split into (pixel, map pair) units,
-    // one warp per map pair, so that it takes a third of a pass.
-    constexpr int kFull = (kP1W * kP1H / kWT) * kWT;
-    constexpr int kRest = kP1W * kP1H - kFull;
-    constexpr int kMP = NW::kM1 / 2;
-    static_assert(kRest <= 32 && 32 * kMP <= kWT, "partial L1 pass must fit one warp per map pair");
-    for (int p = threadIdx.x; p < kFull + 32 * kMP; p += kWT) {
-        const bool unit = p >= kFull;  // one map pair (warp-uniform) of a pixel of the partial pass
-        if (unit && ((p - kFull) & 31) >= kRest) continue;
-        const int px = unit ? kFull + ((p - kFull) & 31) : p;
-        const int mp0 = unit ? (p - kFull) >> 5 : 0;
-        const int x = px % kP1W, y = px / kP1W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < (int)sizeof(S.v.k3) / 16; i += kWT) {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(reinterpret_cast<char*>(S.v.k3) + 16 * i);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(reinterpret_cast<const char*>(G->k3p) + 16 * i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (lane < kInPairs)
+        for (int y = warp; y < kCropH; y += kWT / 32)
+            S.u.in[y][lane & 1][lane >> 1] = make_float2(win_in(S, mode, lane, y), win_in(S, mode, lane + 2 * kHalfW, y));
+    __syncthreads();
+    // L1: conv 4x4 + folded BN/LReLU + 2x2 max, then neighbour sums (add / add2), on the pixels x and x + 11 at
+    // once. 256 pairs take a pass of every map a thread; the last 8 are split into (pair, map) units, one
+    // warp a map, so that they take a sixth of a pass.
+    constexpr int kRest = kP1Pairs - kWT;
+    static_assert(kRest > 0 && kRest <= 32 && NW::kM1 <= kWT / 32, "one full pass, the rest a warp a map");
+    auto pooled = [&](const f2_t (&win)[5][5], int m) {
+        f2_t c[4];
+#pragma unroll
+        for (int k = 0; k < 16; k += 2) {
+            const ulonglong2 w = ld_two(&W.k1d[m][k]);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                const int dy = d >> 1, dx = d & 1;
+                const f2_t a = f2_mul(win[dy + (k >> 2)][dx + (k & 3)], w.x, nz);
+                c[d] = f2_add(k ? f2_add(c[d], a) : a, f2_mul(win[dy + (k >> 2)][dx + (k & 3) + 1], w.y, nz));
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < 4; ++d) c[d] = lrelu_bn2(c[d], W.a1d[m], nz);
+        return f2_max4(c[0], c[1], c[2], c[3]);
+    };
+    auto put = [&](int m, int x, int y, f2_t v) {
+        S.s1[m][y][x] = f2_lo(v);
+        S.s1[m][y][x + kHalfW] = f2_hi(v);
+    };
+    for (int p = threadIdx.x; p < kWT + 32 * NW::kM1; p += kWT) {
+        const bool unit = p >= kWT;  // one map (warp-uniform) of a pair of the partial pass
+        if (unit && lane >= kRest) continue;
+        const int pair = unit ? kWT + lane : p;
+        const int x = pair % kHalfW, y = pair / kHalfW;
         f2_t win[5][5];
 #pragma unroll
         for (int r = 0; r < 5; ++r)
 #pragma unroll
-            for (int c = 0; c < 5; ++c) win[r][c] = f2_dup(win_in(S, mode, 2 * x + c, 2 * y + r));
-        float P[NW::kM1];
-#pragma unroll
-        for (int mp = 0; mp < kMP; ++mp) {
-            if (unit && mp != mp0) continue;
-            f2_t cv[4];
-#pragma unroll
-            for (int d = 0; d < 4; ++d) {
-                const int dy = d >> 1, dx = d & 1;
-                f2_t acc = f2_mul(win[dy][dx], f2_ld(W.k1p[mp][0]), nz);
-#pragma unroll
-                for (int k = 1; k < 16; ++k) acc = f2_add(acc, f2_mul(win[dy + (k >> 2)][dx + (k & 3)], f2_ld(W.k1p[mp][k]), nz));
-                cv[d] = lrelu_bn2(acc, W.a1p[mp], nz);  // maps (2mp, 2mp+1)
-            }
-            const f2_t pm = f2_max4(cv[0], cv[1], cv[2], cv[3]);
-            P[2 * mp] = f2_lo(pm);
-            P[2 * mp + 1] = f2_hi(pm);
-            if (unit) {
-                S.l1rest[px - kFull][2 * mp] = P[2 * mp];
-                S.l1rest[px - kFull][2 * mp + 1] = P[2 * mp + 1];
-            }
+            for (int c = 0; c < 5; ++c) win[r][c] = f2_ld(S.u.in[2 * y + r][c & 1][x + (c >> 1)]);
+        if (unit) {
+            *reinterpret_cast<f2_t*>(&S.l1rest[lane][warp]) = pooled(win, warp);
+            continue;
         }
-        if (unit) continue;
-        S.s1[0][y][x] = fadd(P[0], P[1]);
-#pragma unroll
-        for (int k = 1; k < NW::kM1 - 1; ++k) S.s1[k][y][x] = fadd(fadd(P[k - 1], P[k]), P[k + 1]);
-        S.s1[NW::kM1 - 1][y][x] = fadd(P[NW::kM1 - 2], P[NW::kM1 - 1]);
+        f2_t before = 0ull, last = pooled(win, 0);  // maps m - 2 and m - 1
+#pragma unroll 1
+        for (int m = 1; m < NW::kM1; ++m) {
+            const f2_t v = pooled(win, m);
+            const f2_t two = m == 1 ? last : f2_add(before, last);
+            put(m - 1, x, y, f2_add(two, v));
+            before = last;
+            last = v;
+        }
+        put(NW::kM1 - 1, x, y, f2_add(before, last));
     }
-    if (kRest > 0) {
-        __syncthreads();
-        if (threadIdx.x < kRest) {
-            const int px = kFull + threadIdx.x;
-            const int x = px % kP1W, y = px / kP1W;
-            const float* P = S.l1rest[threadIdx.x];
-            S.s1[0][y][x] = fadd(P[0], P[1]);
+    __syncthreads();
+    if (threadIdx.x < kRest) {
+        const int x = (kWT + threadIdx.x) % kHalfW, y = (kWT + threadIdx.x) / kHalfW;
+        f2_t P[NW::kM1];
 #pragma unroll
-            for (int k = 1; k < NW::kM1 - 1; ++k) S.s1[k][y][x] = fadd(fadd(P[k - 1], P[k]), P[k + 1]);
-            S.s1[NW::kM1 - 1][y][x] = fadd(P[NW::kM1 - 2], P[NW::kM1 - 1]);
-        }
+        for (int k = 0; k < NW::kM1; ++k) P[k] = f2_ld(S.l1rest[threadIdx.x][k]);
+        put(0, x, y, f2_add(P[0], P[1]));
+#pragma unroll
+        for (int k = 1; k < NW::kM1 - 1; ++k) put(k, x, y, f2_add(f2_add(P[k - 1], P[k]), P[k + 1]));
+        put(NW::kM1 - 1, x, y, f2_add(P[NW::kM1 - 2], P[NW::kM1 - 1]));
     }
     __syncthreads();
     // L2: map pair (2i, 2i+1) convolves sum map i; 3x3 + BN/LReLU + 2x2 max
@@ -125,38 +165,42 @@ __device__ void window_net(const NW& W, WindowSmem& S, int mode) {
             for (int c = 0; c < 4; ++c) q[r][c] = f2_dup(S.s1[i][2 * y + r][2 * x + c]);
         f2_t cv[4];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const int dy = d >> 1, dx = d & 1;
-            f2_t acc = f2_mul(q[dy][dx], f2_ld(W.k2p[i][0]), nz);
+        for (int k = 0; k < 9; ++k) {
+            const f2_t w = f2_ld(W.k2p[i][k]);
 #pragma unroll
-            for (int k = 1; k < 9; ++k) acc = f2_add(acc, f2_mul(q[dy + k / 3][dx + k % 3], f2_ld(W.k2p[i][k]), nz));
-            cv[d] = lrelu_bn2(acc, W.a2p[i], nz);
+            for (int d = 0; d < 4; ++d) {
+                const f2_t a = f2_mul(q[(d >> 1) + k / 3][(d & 1) + k % 3], w, nz);
+                cv[d] = k ? f2_add(cv[d], a) : a;
+            }
         }
+#pragma unroll
+        for (int d = 0; d < 4; ++d) cv[d] = lrelu_bn2(cv[d], W.a2p[i], nz);
         const f2_t pm = f2_max4(cv[0], cv[1], cv[2], cv[3]);
-        S.p2[2 * i][y][x] = f2_lo(pm);
-        S.p2[2 * i + 1][y][x] = f2_hi(pm);
+        S.u.l.p2[2 * i][y][x] = f2_lo(pm);
+        S.u.l.p2[2 * i + 1][y][x] = f2_hi(pm);
     }
     __syncthreads();
     for (int p = threadIdx.x; p < kP2W * kP2H; p += kWT) {
         const int x = p % kP2W, y = p / kP2W;
         constexpr int M = NW::kM2;
-        S.s2[0][y][x] = fadd(S.p2[0][y][x], S.p2[1][y][x]);
-        for (int k = 1; k < M - 1; ++k) S.s2[k][y][x] = fadd(fadd(S.p2[k - 1][y][x], S.p2[k][y][x]), S.p2[k + 1][y][x]);
-        S.s2[M - 1][y][x] = fadd(S.p2[M - 2][y][x], S.p2[M - 1][y][x]);
+        S.u.l.s2[0][y][x] = fadd(S.u.l.p2[0][y][x], S.u.l.p2[1][y][x]);
+        for (int k = 1; k < M - 1; ++k) S.u.l.s2[k][y][x] = fadd(fadd(S.u.l.p2[k - 1][y][x], S.u.l.p2[k][y][x]), S.u.l.p2[k + 1][y][x]);
+        S.u.l.s2[M - 1][y][x] = fadd(S.u.l.p2[M - 2][y][x], S.u.l.p2[M - 1][y][x]);
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     // L3: 7w x 8h conv summed in one left-to-right chain (conv_8x7), BN/LReLU, no pooling;
     // maps (2i, 2i+1) share the input: packed
     for (int it = threadIdx.x; it < (NW::kM3 / 2) * kOutN; it += kWT) {
         const int i = it / kOutN, o = it - i * kOutN;
         const int ox = o & 3, oy = o >> 2;
-        f2_t acc = f2_mul(f2_dup(S.s2[i][oy][ox]), f2_ld(W.k3p[i][0]), nz);
+        f2_t acc = f2_mul(f2_dup(S.u.l.s2[i][oy][ox]), f2_ld(S.v.k3[i][0]), nz);
 #pragma unroll
         for (int k = 1; k < NW::kK3W * NW::kK3H; ++k)
-            acc = f2_add(acc, f2_mul(f2_dup(S.s2[i][oy + k / NW::kK3W][ox + k % NW::kK3W]), f2_ld(W.k3p[i][k]), nz));
-        const f2_t av = lrelu_bn2(acc, W.a3p[i], nz);
-        S.a3[2 * i][o] = f2_lo(av);
-        S.a3[2 * i + 1][o] = f2_hi(av);
+            acc = f2_add(acc, f2_mul(f2_dup(S.u.l.s2[i][oy + k / NW::kK3W][ox + k % NW::kK3W]), f2_ld(S.v.k3[i][k]), nz));
+        const f2_t av = lrelu_bn2(acc, G->a3p[i], nz);
+        S.u.l.a3[2 * i][o] = f2_lo(av);
+        S.u.l.a3[2 * i + 1][o] = f2_hi(av);
     }
     __syncthreads();
     // hidden neurons n = HS*i + t read L3 maps i .. i+CONN-1; neurons (2q, 2q+1) share the
@@ -165,22 +209,22 @@ __device__ void window_net(const NW& W, WindowSmem& S, int mode) {
         const int q = it / kOutN, o = it - q * kOutN;
         const int n = 2 * q;
         const int i = n / NW::kHS;
-        f2_t s = f2_pack(W.hb[n], W.hb[n + 1]);
+        f2_t s = f2_pack(__ldg(&G->hb[n]), __ldg(&G->hb[n + 1]));
 #pragma unroll
-        for (int j = 0; j < NW::kConn; ++j) s = f2_add(s, f2_mul(f2_dup(S.a3[i + j][o]), f2_ld(W.hwp[q][j]), nz));
-        s = f2_mul(s, f2_dup(W.htw[i]), nz);
+        for (int j = 0; j < NW::kConn; ++j) s = f2_add(s, f2_mul(f2_dup(S.u.l.a3[i + j][o]), f2_ld(G->hwp[q][j]), nz));
+        s = f2_mul(s, f2_dup(__ldg(&G->htw[i])), nz);
         const f2_t half = f2_pack(0.5f, 0.5f);
         const f2_t v = f2_add(f2_mul(half, tanh_rational2(s, nz), nz), half);
         const int t = n - i * NW::kHS;  // neurons n, n+1 are slots t, t+1 of group i
-        const f2_t h = f2_add(f2_mul(f2_pack(W.hbnw[t], W.hbnw[t + 1]), v, nz), f2_pack(W.hbnb[t], W.hbnb[t + 1]));
-        S.hbuf[n][o] = f2_lo(h);
-        S.hbuf[n + 1][o] = f2_hi(h);
+        const f2_t h = f2_add(f2_mul(f2_pack(__ldg(&G->hbnw[t]), __ldg(&G->hbnw[t + 1])), v, nz), f2_pack(__ldg(&G->hbnb[t]), __ldg(&G->hbnb[t + 1])));
+        S.v.hbuf[n][o] = f2_lo(h);
+        S.v.hbuf[n + 1][o] = f2_hi(h);
     }
     __syncthreads();
     if (threadIdx.x < kOutN) {
         const int o = threadIdx.x;
-        float acc = fmul(S.hbuf[0][o], W.ow[0]);
-        for (int n = 1; n < NW::kHL; ++n) acc = fadd(fmul(S.hbuf[n][o], W.ow[n]), acc);
+        float acc = fmul(S.v.hbuf[0][o], W.ow[0]);
+        for (int n = 1; n < NW::kHL; ++n) acc = fadd(fmul(S.v.hbuf[n][o], W.ow[n]), acc);
         float c = fmul(fadd(acc, W.ob), W.otw);
         c = tanh_rational(c);
         S.out[o] = (W.af == 0.f) ? fadd(fmul(0.5f, c), 0.5f) : fmul(W.af, c);
@@ -237,8 +281,7 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
             P[2 * mp] = f2_lo(v);
             P[2 * mp + 1] = f2_hi(v);
             if (unit) {
-                S.l1rest[px - kFull][2 * mp] = P[2 * mp];
-                S.l1rest[px - kFull][2 * mp + 1] = P[2 * mp + 1];
+                S.l1rest[px - kFull][mp] = make_float2(P[2 * mp], P[2 * mp + 1]);
             }
         }
         if (!unit) sums(P, px);
@@ -247,7 +290,7 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
     if (threadIdx.x < kRest) {
         float P[kM0];
 #pragma unroll
-        for (int k = 0; k < kM0; ++k) P[k] = S.l1rest[threadIdx.x][k];
+        for (int k = 0; k < kM0; ++k) P[k] = (k & 1) ? S.l1rest[threadIdx.x][k / 2].y : S.l1rest[threadIdx.x][k / 2].x;
         sums(P, kFull + threadIdx.x);
     }
     __syncthreads();
@@ -270,15 +313,15 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
             }
         }
         const f2_t v = lg_pool_tanh2(c, W.max_pool, lg_pool_pair(W, 1, i), af, nz);
-        S.p2[2 * i][y][x] = f2_lo(v);
-        S.p2[2 * i + 1][y][x] = f2_hi(v);
+        S.u.l.p2[2 * i][y][x] = f2_lo(v);
+        S.u.l.p2[2 * i + 1][y][x] = f2_hi(v);
     }
     __syncthreads();
     for (int it = threadIdx.x; it < W.m1 * kP2; it += kWT) {
         const int k = it / kP2, p = it - k * kP2;
         const int x = p % kP2W, y = p / kP2W;
-        const float two = k ? fadd(S.p2[k - 1][y][x], S.p2[k][y][x]) : fadd(S.p2[0][y][x], S.p2[1][y][x]);
-        S.s2[k][y][x] = (k == 0 || k == W.m1 - 1) ? two : fadd(two, S.p2[k + 1][y][x]);
+        const float two = k ? fadd(S.u.l.p2[k - 1][y][x], S.u.l.p2[k][y][x]) : fadd(S.u.l.p2[0][y][x], S.u.l.p2[1][y][x]);
+        S.u.l.s2[k][y][x] = (k == 0 || k == W.m1 - 1) ? two : fadd(two, S.u.l.p2[k + 1][y][x]);
     }
     __syncthreads();
     constexpr int kK3W = 7, kK3H = 8;  // the third-layer kernel of the stage-2/3 networks
@@ -288,18 +331,18 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
         f2_t acc = 0ull;
 #pragma unroll
         for (int t = 0; t < kK3W * kK3H; ++t) {
-            const f2_t m = f2_mul(f2_dup(S.s2[i][oy + t / kK3W][ox + t % kK3W]), f2_pack(__ldg(&W.k3[2 * i][t]), __ldg(&W.k3[2 * i + 1][t])), nz);
+            const f2_t m = f2_mul(f2_dup(S.u.l.s2[i][oy + t / kK3W][ox + t % kK3W]), f2_pack(__ldg(&W.k3[2 * i][t]), __ldg(&W.k3[2 * i + 1][t])), nz);
             acc = t ? f2_add(acc, m) : m;
         }
         const f2_t v = lg_l3_finish2(W, lg_l3_pair(W, i), acc, nz);
-        S.a3[2 * i][o] = f2_lo(v);
-        S.a3[2 * i + 1][o] = f2_hi(v);
+        S.u.l.a3[2 * i][o] = f2_lo(v);
+        S.u.l.a3[2 * i + 1][o] = f2_hi(v);
     }
     __syncthreads();
     if (W.full_connect) {
         for (int it = threadIdx.x; it < W.hl * kOutN; it += kWT) {
             const int n = it / kOutN, o = it - n * kOutN;
-            S.hbuf[n][o] = lg_hidden_fc(W, n, [&](int j) { return S.a3[j][o]; });
+            S.v.hbuf[n][o] = lg_hidden_fc(W, n, [&](int j) { return S.u.l.a3[j][o]; });
         }
         __syncthreads();
     }
@@ -307,11 +350,11 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
         const int o = threadIdx.x;
         float acc;
         if (W.full_connect) {
-            acc = S.hbuf[0][o];
-            for (int n = 1; n < W.hl; ++n) acc = fadd(acc, S.hbuf[n][o]);
+            acc = S.v.hbuf[0][o];
+            for (int n = 1; n < W.hl; ++n) acc = fadd(acc, S.v.hbuf[n][o]);
         } else {
-            acc = fadd(S.a3[1][o], S.a3[0][o]);
-            for (int i = 1; i < W.m2 / 2; ++i) acc = fadd(acc, fadd(S.a3[2 * i + 1][o], S.a3[2 * i][o]));
+            acc = fadd(S.u.l.a3[1][o], S.u.l.a3[0][o]);
+            for (int i = 1; i < W.m2 / 2; ++i) acc = fadd(acc, fadd(S.u.l.a3[2 * i + 1][o], S.u.l.a3[2 * i][o]));
         }
         S.out[o] = lg_finish(W, acc);
     }
@@ -326,6 +369,7 @@ struct WinArgs {
     const LevelDesc* levels;
     WinOut* out;
     CascadeConfig cfg;
+    const WindowNets* nets;  // the CNTK networks in device memory too
     const LegacyNet* lg;  // legacy networks ([1] stage 2, [2] stage 3) instead of the CNTK ones, or null
     float2 negzero;       // (-0, -0), for the legacy networks (the CNTK ones carry their own)
 };
@@ -338,52 +382,49 @@ __device__ void prepare_window(const WinArgs& a, WindowSmem& S, const Candidate&
     const int rx = S.geo[0], ry = S.geo[1], rcols = S.geo[2], rrows = S.geo[3];
     const bool copy = (rcols == kCropW && rrows == kCropH);  // FastImageResize copies equal sizes
     const uint32_t sclx = fp_step(max(rcols, 1), kCropW), scly = fp_step(max(rrows, 1), kCropH);
-    // every load of the thread's pixels is issued before the first is used (the gray frame is read
-    // from L2, so the loads overlap instead of queueing one latency each); the byte values stay in
-    // registers until the equalisation table is known
-    constexpr int kPx = kCropW * kCropH;
-    constexpr int kPerThread = (kPx + kWT - 1) / kWT;
-    float v[kPerThread];
+    // a warp a row, a lane the columns lane and lane + 32. Every load of a thread's pixels is issued before the first
+    // is used (the gray frame is read from L2, so the loads overlap instead of queueing one latency each);
+    // the byte values stay in registers until the equalisation table is known
+    constexpr int kRows = (kCropH + kWT / 32 - 1) / (kWT / 32);  // 7 rows a warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool two = lane + 32 < kCropW;
+    // the clamps are memory guards only: valid candidates always sample inside the frame
+    int gx[2];
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int p = threadIdx.x + k * kWT;
-        v[k] = 0.f;
-        if (p < kPx) {
-            const int ix = p % kCropW, iy = p / kCropW;
-            int sx, sy;
-            if (copy) {
-                sx = ix;
-                sy = iy;
-            } else {
-                sx = (int)sample_col(ix, sclx, rcols).idx;
-                sy = (int)sample_row(iy, scly, rrows).idx;
-            }
-            // memory guard only: valid candidates always sample inside the frame
-            const int gx = min(max(rx + sx, 0), a.gw - 1), gy = min(max(ry + sy, 0), a.gh - 1);
-            v[k] = a.gray[(size_t)gy * a.gpitch + gx];
-        }
+    for (int h = 0; h < 2; ++h) {
+        const int ix = min(lane + 32 * h, kCropW - 1);
+        gx[h] = min(max(rx + (copy ? ix : (int)sample_col(ix, sclx, rcols).idx), 0), a.gw - 1);
+    }
+    float v[kRows][2];
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+        const int iy = min(warp + k * (kWT / 32), kCropH - 1);
+        const int gy = min(max(ry + (copy ? iy : (int)sample_row(iy, scly, rrows).idx), 0), a.gh - 1);
+        const float* row = a.gray + (size_t)gy * a.gpitch;
+        v[k][0] = row[gx[0]];
+        v[k][1] = two ? row[gx[1]] : 0.f;
     }
     const bool eq = a.cfg.equalize != 0;
-    uint32_t u[(kPerThread + 3) / 4];  // the bytes, four to a register
+    uint32_t u[(2 * kRows + 3) / 4];  // the bytes, four to a register
 #pragma unroll
-    for (int k = 0; k < (kPerThread + 3) / 4; ++k) u[k] = 0u;
+    for (int k = 0; k < (2 * kRows + 3) / 4; ++k) u[k] = 0u;
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int p = threadIdx.x + k * kWT;
-        const uint32_t b = (uint8_t)__float2int_rz(fadd(v[k], 0.5f));
-        u[k >> 2] |= b << (8 * (k & 3));
-        if (p < kPx) {
+    for (int q = 0; q < 2 * kRows; ++q) {
+        const int iy = warp + (q >> 1) * (kWT / 32), ix = lane + 32 * (q & 1);
+        const uint32_t b = (uint8_t)__float2int_rz(fadd(v[q >> 1][q & 1], 0.5f));
+        u[q >> 2] |= b << (8 * (q & 3));
+        if (iy < kCropH && ix < kCropW) {
             if (eq)
                 atomicAdd(&S.hist[b], 1);
             else
-                S.crop[p / kCropW][p % kCropW] = (uint8_t)b;
+                S.crop[iy][ix] = (uint8_t)b;
         }
     }
     __syncthreads();
     if (!eq) return;
     // cumulative histogram (256 bins, one per thread): shuffle scan + warp totals
     {
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        const int wid = warp;
         int c = S.hist[threadIdx.x];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -408,10 +449,10 @@ __device__ void prepare_window(const WinArgs& a, WindowSmem& S, const Candidate&
     }
     // the equalised bytes (the reference leaves the window unchanged when every pixel is equal)
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int p = threadIdx.x + k * kWT;
-        const uint32_t b = (u[k >> 2] >> (8 * (k & 3))) & 0xffu;
-        if (p < kPx) S.crop[p / kCropW][p % kCropW] = (uint8_t)(bmin != bmax ? S.lut[b] : b);
+    for (int q = 0; q < 2 * kRows; ++q) {
+        const int iy = warp + (q >> 1) * (kWT / 32), ix = lane + 32 * (q & 1);
+        const uint32_t b = (u[q >> 2] >> (8 * (q & 3))) & 0xffu;
+        if (iy < kCropH && ix < kCropW) S.crop[iy][ix] = (uint8_t)(bmin != bmax ? S.lut[b] : b);
     }
     __syncthreads();
 }
@@ -439,9 +480,9 @@ __device__ __forceinline__ void window_item(const WindowNets& N, const WinArgs& 
         if constexpr (kLegacy)
             legacy_window_net(a.lg[1 + stage], S, stage == 0 ? 0 : (C.reflection ? 1 : 2), f2_ld(a.negzero));
         else if (stage == 0)
-            window_net(N.s2, S, 0);
+            window_net(N.s2, &a.nets->s2, S, 0);
         else
-            window_net(N.s3, S, C.reflection ? 1 : 2);
+            window_net(N.s3, &a.nets->s3, S, C.reflection ? 1 : 2);
         // every thread reduces the 16 responses itself (no extra barrier needed)
         const float thr = stage == 0 ? C.thr2 : C.thr3;
         float mx = -10.f;
@@ -512,7 +553,7 @@ __global__ void __launch_bounds__(kWT, kMinBlocks) window_batch_kernel(const __g
 
 int window_smem_bytes() { return (int)sizeof(WindowSmem); }
 
-cudaError_t launch_window_batch(const WindowNets& N, const WinBatch& B, int gpitch, int gw, int gh, const LevelDesc* levels,
+cudaError_t launch_window_batch(const WindowNets& N, const WindowNets* d_nets, const WinBatch& B, int gpitch, int gw, int gh, const LevelDesc* levels,
                                 const CascadeConfig& cfg, int grid, cudaStream_t st, int ctas_per_sm) {
     WinArgs a{};
     a.gpitch = gpitch;
@@ -521,6 +562,7 @@ cudaError_t launch_window_batch(const WindowNets& N, const WinBatch& B, int gpit
     a.levels = levels;
     a.cfg = cfg;
     a.lg = nullptr;
+    a.nets = d_nets;
     if (ctas_per_sm <= 2)
         window_batch_kernel<2><<<grid, kWT, sizeof(WindowSmem), st>>>(N, a, B);
     else
@@ -528,7 +570,7 @@ cudaError_t launch_window_batch(const WindowNets& N, const WinBatch& B, int gpit
     return cudaGetLastError();
 }
 
-cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, int gw, int gh, const Candidate* cands, const int* n_cand,
+cudaError_t launch_window(const WindowNets& N, const WindowNets* d_nets, const float* gray, int gpitch, int gw, int gh, const Candidate* cands, const int* n_cand,
                           const LevelDesc* levels, WinOut* out, const CascadeConfig& cfg, int grid, cudaStream_t st, const LegacyNet* lg,
                           int ctas_per_sm) {
     static_assert(sizeof(WindowSmem) + 64 <= 48 * 1024, "window kernel shared memory must stay under the default 48 KB");
@@ -543,6 +585,7 @@ cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, in
     a.out = out;
     a.cfg = cfg;
     a.lg = lg;
+    a.nets = d_nets;
     a.negzero = make_float2(-0.f, -0.f);
     const auto kernel = lg ? (ctas_per_sm <= 2 ? window_kernel<true, 2> : window_kernel<true, 4>)
                         : ctas_per_sm <= 2 ? window_kernel<false, 2>

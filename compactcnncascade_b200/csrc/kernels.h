@@ -184,7 +184,7 @@ struct WinBatch {
     WinOut* out[kMaxBatch];
     int n_frames;
 };
-cudaError_t launch_window_batch(const WindowNets& N, const WinBatch& B, int gpitch, int gw, int gh, const LevelDesc* levels,
+cudaError_t launch_window_batch(const WindowNets& N, const WindowNets* d_nets, const WinBatch& B, int gpitch, int gw, int gh, const LevelDesc* levels,
                                 const CascadeConfig& cfg, int grid, cudaStream_t st, int ctas_per_sm = 4);
 // the replay of every frame of a batch: block f runs args[f] (device memory)
 cudaError_t launch_replay_batch(const ReplayArgs* d_args, int n_frames, cudaStream_t st);
@@ -224,11 +224,11 @@ cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_
                                Stage1Sched sched = Stage1Sched{});
 cudaError_t launch_cand_write(const int4* d_chunks, int n_chunks, const LevelDesc* d_levels, const float* resp, float thr,
                               const int* counts, Candidate* out, int* n_out, int cap, cudaStream_t st);
-// lg (optional): the legacy networks (device memory, [1] stage 2, [2] stage 3) replace N
+// d_nets: N in device memory too (16-byte aligned). lg (optional): the legacy networks (device memory, [1] stage 2, [2] stage 3) replace N
 // ctas_per_sm: resident blocks a SM the grid was sized for (1-6); 2 or fewer selects the
 // 128-register build, 5 and 6 the 48- and 40-register ones
 cudaError_t window_setup();
-cudaError_t launch_window(const WindowNets& N, const float* gray, int gpitch, int gw, int gh, const Candidate* cands, const int* n_cand,
+cudaError_t launch_window(const WindowNets& N, const WindowNets* d_nets, const float* gray, int gpitch, int gw, int gh, const Candidate* cands, const int* n_cand,
                           const LevelDesc* levels, WinOut* out, const CascadeConfig& cfg, int grid, cudaStream_t st,
                           const LegacyNet* lg = nullptr, int ctas_per_sm = 4);
 // one legacy (format 1.0) network on each of the levels; counts (optional) gets each scan chunk's responses
