@@ -11,8 +11,8 @@
 //        rows of a strip of two pooled rows and runs on its own), runs the 4x4 conv + folded
 //        BN/LReLU + 2x2 max for the 4 L1 maps and writes the 4 neighbour-map sums that L2 consumes
 //        (S1 arena). Bound by the fp32 pipe (65 % busy; about 87 % is what these packed chains reach
-//        alone) and the latency of the gray samples: 1.09 ms for the 83 levels of a 3840x2160 frame at
-//        scale 1.05 (1.30 with 256-thread blocks and 25 % more instructions: the row references once a
+//        alone) and the latency of the gray samples: 1.06 ms for the 83 levels of a 3840x2160 frame at
+//        scale 1.05 (1.09 with one weight a constant load instead of two, 1.30 with 256-thread blocks and 25 % more instructions: the row references once a
 //        tile instead of once a sample, both gray rows of a sample as one packed chain), 39.8 us for the
 //        13 of a 1080p frame (43.3).
 // back:  one CTA per 32x16 tile of response pixels (128 threads with two pixel pairs a thread, 256 with
@@ -101,6 +101,15 @@ struct alignas(16) RowRef {
     float pad;
     float2 cf;
 };
+
+// Two consecutive duplicated parameters by one 16-byte constant load.
+struct Pair16 {
+    f2_t a, b;
+};
+__device__ __forceinline__ Pair16 ld_pair(const float2* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return Pair16{v.x, v.y};
+}
 
 struct FrontSmem {
     union {
@@ -265,13 +274,17 @@ __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const
         for (int m = 0; m < 4; ++m) {
             f2_t cv[4];
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-                const int dy = d >> 1, dx = d & 1;
-                f2_t acc = f2_mul(pr[dy][dx], f2_ld(W.k1d[m][0]), nz);
+            for (int k = 0; k < 16; k += 2) {
+                const Pair16 w = ld_pair(&W.k1d[m][k]);
 #pragma unroll
-                for (int k = 1; k < 16; ++k) acc = f2_add(acc, f2_mul(pr[dy + (k >> 2)][dx + (k & 3)], f2_ld(W.k1d[m][k]), nz));
-                cv[d] = lrelu_bn2(acc, W.a1d[m], nz);
+                for (int d = 0; d < 4; ++d) {
+                    const int dy = d >> 1, dx = d & 1;
+                    const f2_t a = f2_mul(pr[dy + (k >> 2)][dx + (k & 3)], w.a, nz);
+                    cv[d] = f2_add(k ? f2_add(cv[d], a) : a, f2_mul(pr[dy + (k >> 2)][dx + (k & 3) + 1], w.b, nz));
+                }
             }
+#pragma unroll
+            for (int d = 0; d < 4; ++d) cv[d] = lrelu_bn2(cv[d], W.a1d[m], nz);
             P[m] = f2_max4(cv[0], cv[1], cv[2], cv[3]);
         }
         // neighbour-map sums consumed by L2 (add/add2 of the reference)
@@ -415,14 +428,6 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Two consecutive duplicated parameters by one 16-byte constant load.
-struct Pair16 {
-    f2_t a, b;
-};
-__device__ __forceinline__ Pair16 ld_pair(const float2* p) {
-    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-    return Pair16{v.x, v.y};
-}
 __device__ __forceinline__ f2_t lrelu_bn_d(f2_t x, const float2* p, f2_t nz) {
     const Pair16 u = ld_pair(p), v = ld_pair(p + 2);
     const f2_t c = f2_add(x, u.a);
@@ -460,7 +465,7 @@ __device__ __forceinline__ f2_t pool_l2(const f2_t (*q)[4], const Stage1Back::L2
 //      are now known (the two partial sums a pixel still needs stay in registers);
 //   C: the L3 maps (4w x 5h) of those sums, the hidden groups whose four L3 maps are now known and their
 //      part of the output sum, all in registers, while S1 map k + 1 is copied (cp.async).
-// Only one S1 map and three sums are ever held, 21 KB, so that registers alone limit the resident blocks.
+// Two S1 maps and three sums are ever held, 33 KB, so that registers alone limit the resident blocks.
 // Back tile t of level L as above; g is its global back-tile index (the gate's tile index).
 // kCoherent: the S1 arena was written earlier in the same launch (read through L2).
 // Warps (32 x 2 kPairs response pixels) and L2 rows that only pixels past the map's last row need are
