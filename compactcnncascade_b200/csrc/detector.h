@@ -105,7 +105,7 @@ class Detector {
    public:
     static constexpr int kSlots = 8;
     static constexpr int kHostFaces = 1024;
-    static constexpr int kGraphFaces = 64;  // faces each frame's graph downloads; more are fetched on demand
+    static constexpr int kGraphFaces = 64;  // faces a frame that a batch's graph downloads; more are fetched on demand
 
     Detector() = default;
     ~Detector();

@@ -11,10 +11,10 @@
 //        rows of a strip of two pooled rows and runs on its own), runs the 4x4 conv + folded
 //        BN/LReLU + 2x2 max for the 4 L1 maps and writes the 4 neighbour-map sums that L2 consumes
 //        (S1 arena). Bound by the fp32 pipe (65 % busy; about 87 % is what these packed chains reach
-//        alone) and the latency of the gray samples: 1.06 ms for the 83 levels of a 3840x2160 frame at
-//        scale 1.05 (1.09 with one weight a constant load instead of two, 1.30 with 256-thread blocks and 25 % more instructions: the row references once a
-//        tile instead of once a sample, both gray rows of a sample as one packed chain), 39.8 us for the
-//        13 of a 1080p frame (43.3).
+//        alone) and the latency of the gray samples: 1.09 ms for the 83 levels of a 3840x2160 frame at
+//        scale 1.05 (1.30 with 256-thread blocks and 25 % more instructions: the row references once a tile
+//        instead of once a sample, both gray rows of a sample as one packed chain), 39.8 us for the 13 of a
+//        1080p frame (43.3); two weights a constant load instead of one took 3 % more off.
 // back:  one CTA per 32x16 tile of response pixels (128 threads with two pixel pairs a thread, 256 with
 //        one). It takes the S1 tile (4 x 42 x 72) map by map through two shared-memory buffers
 //        (asynchronous copies), computes the pooled L2 maps of each and the sums they complete on the
