@@ -167,10 +167,8 @@ struct NetWeights {
     static constexpr int kK1W = K1W, kK1H = K1H, kK2W = K2W, kK2H = K2H, kK3W = K3W, kK3H = K3H;
     static constexpr int kHL = HL, kConn = CONN, kHS = HS, kGroups = HL / HS;
     alignas(16) float2 k1d[M1][K1W * K1H];  // L1 taps duplicated (w, w): two pixels of one map per packed op
-    float2 k1p[M1 / 2][K1W * K1H];  // L1 taps of maps (2i, 2i+1), which read the same input
     float b1[M1], w1a[M1], w1b[M1], bn1[M1];
     float2 a1d[M1][4];              // L1 {b, w1a, w1b, bn} of each map duplicated (v, v)
-    float2 a1p[M1 / 2][4];          // L1 {b, w1a, w1b, bn} of map pairs (2i, 2i+1)
     float2 k2p[M2 / 2][K2W * K2H];  // L2 taps of maps (2i, 2i+1), which read the same sum map i
     float b2[M2], w2a[M2], w2b[M2], bn2[M2];
     float2 a2p[M2 / 2][4];          // L2 {b, w2a, w2b, bn} of map pairs

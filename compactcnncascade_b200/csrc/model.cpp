@@ -137,8 +137,6 @@ bool pack_model(const RawModel& m, int index_output, NW* o, std::string* err) {
     auto tap = [&](int l, int mm, int k) { return m.kernels[l][(size_t)mm * m.kw[l] * m.kh[l] + k]; };
     for (int mm = 0; mm < NW::kM1; ++mm)
         for (int k = 0; k < NW::kK1W * NW::kK1H; ++k) o->k1d[mm][k] = make_float2(tap(0, mm, k), tap(0, mm, k));
-    for (int i = 0; i < NW::kM1 / 2; ++i)
-        for (int k = 0; k < NW::kK1W * NW::kK1H; ++k) o->k1p[i][k] = make_float2(tap(0, 2 * i, k), tap(0, 2 * i + 1, k));
     for (int i = 0; i < NW::kM2 / 2; ++i)
         for (int k = 0; k < NW::kK2W * NW::kK2H; ++k) o->k2p[i][k] = make_float2(tap(1, 2 * i, k), tap(1, 2 * i + 1, k));
     for (int i = 0; i < NW::kM3 / 2; ++i)
@@ -165,12 +163,6 @@ bool pack_model(const RawModel& m, int index_output, NW* o, std::string* err) {
     for (int mm = 0; mm < NW::kM1; ++mm) {
         const float v[4] = {o->b1[mm], o->w1a[mm], o->w1b[mm], o->bn1[mm]};
         for (int f = 0; f < 4; ++f) o->a1d[mm][f] = make_float2(v[f], v[f]);
-    }
-    for (int i = 0; i < NW::kM1 / 2; ++i) {
-        o->a1p[i][0] = make_float2(o->b1[2 * i], o->b1[2 * i + 1]);
-        o->a1p[i][1] = make_float2(o->w1a[2 * i], o->w1a[2 * i + 1]);
-        o->a1p[i][2] = make_float2(o->w1b[2 * i], o->w1b[2 * i + 1]);
-        o->a1p[i][3] = make_float2(o->bn1[2 * i], o->bn1[2 * i + 1]);
     }
     for (int i = 0; i < NW::kM2 / 2; ++i) {
         o->a2p[i][0] = make_float2(o->b2[2 * i], o->b2[2 * i + 1]);
