@@ -292,7 +292,7 @@ __host__ __device__ __forceinline__ int gate_cell_lo(int p, int m) { return (p -
 __host__ __device__ __forceinline__ int gate_cell_hi(int p, int m, int n16) { return (p + m) / 16 < n16 - 1 ? (p + m) / 16 : n16 - 1; }
 
 // any set bit of octave row bitmaps `B` in cells [cx0, cx1] x [cy0, cy1]
-__device__ __forceinline__ bool gate_any_bit(const uint32_t* __restrict__ B, int wwords, int cx0, int cx1, int cy0, int cy1) {
+__device__ __forceinline__ bool gate_any_bit(const uint32_t* B, int wwords, int cx0, int cx1, int cy0, int cy1) {
     if (cx0 > cx1 || cy0 > cy1) return false;
     const int w0 = cx0 >> 5, w1 = cx1 >> 5;
     const uint32_t m0 = 0xffffffffu << (cx0 & 31), m1 = 0xffffffffu >> (31 - (cx1 & 31));

@@ -162,9 +162,8 @@ __device__ __forceinline__ void centre_cells(const LevelDesc& L, int ox0, int ox
 // kMaskSmemWords read them from global memory.
 constexpr int kMaskSmemWords = 12288;
 
-__global__ void gate_mask_kernel(const __grid_constant__ LevelTable LT, int nb, const uint32_t* __restrict__ gbits, int n_words, int wwords,
-                                 int w16, int h16, int margin, const int* __restrict__ ambiguous, int amb_limit, uint8_t* __restrict__ back_on,
-                                 uint8_t* __restrict__ front_on) {
+__global__ void gate_mask_kernel(const __grid_constant__ LevelTable LT, int nb, const uint32_t* gbits, int n_words, int wwords, int w16, int h16,
+                                 int margin, const int* ambiguous, int amb_limit, uint8_t* back_on, uint8_t* front_on) {
     extern __shared__ uint32_t sbits[];
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

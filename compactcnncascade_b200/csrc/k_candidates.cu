@@ -36,8 +36,7 @@ constexpr int kChunkRounds = kCandChunk / kChunkThreads;  // 8
 static_assert(kChunkRounds * kChunkThreads == kCandChunk, "a chunk is whole rounds of the block");
 
 __device__ __forceinline__ void cand_write_chunk(const int4* __restrict__ chunks, int n_chunks, const LevelDesc* __restrict__ levels,
-                                                 const float* __restrict__ resp, float thr, const int* __restrict__ counts,
-                                                 Candidate* __restrict__ out, int* __restrict__ n_out, int cap, int c) {
+                                                 const float* resp, float thr, const int* counts, Candidate* out, int* n_out, int cap, int c) {
     __shared__ int wt[32];
     __shared__ int rw[kChunkRounds * (kChunkThreads / 32)];
     const int hits = counts[c];  // uniform over the block
@@ -87,9 +86,8 @@ __device__ __forceinline__ void cand_write_chunk(const int4* __restrict__ chunks
 }
 
 __global__ void __launch_bounds__(kChunkThreads) cand_write_kernel(const int4* __restrict__ chunks, int n_chunks,
-                                                                   const LevelDesc* __restrict__ levels, const float* __restrict__ resp,
-                                                                   float thr, const int* __restrict__ counts, Candidate* __restrict__ out,
-                                                                   int* __restrict__ n_out, int cap) {
+                                                                   const LevelDesc* __restrict__ levels, const float* resp, float thr,
+                                                                   const int* counts, Candidate* out, int* n_out, int cap) {
     chain_wait();
     cand_write_chunk(chunks, n_chunks, levels, resp, thr, counts, out, n_out, cap, blockIdx.x);
 }

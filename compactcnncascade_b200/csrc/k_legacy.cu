@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kLgT) legacy_pool_kernel(const LegacyNet* __re
 #pragma unroll
         for (int r = 0; r < 5; ++r)
 #pragma unroll
-            for (int c = 0; c < 5; ++c) win[r][c] = f2_dup(__ldg(src + (size_t)r * V.L.pitch + c));
+            for (int c = 0; c < 5; ++c) win[r][c] = f2_dup(ld_chain(src + (size_t)r * V.L.pitch + c));
         float P[kLgMaxM0];
 #pragma unroll
         for (int p = 0; p < kLgMaxM0 / 2; ++p) {
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kLgT) legacy_pool_kernel(const LegacyNet* __re
 // loaded once and continues the chains of the rows that it reaches (each output's taps stay in row-major
 // order); the pair's weights are in registers. done(row, (c0, c1)) takes each result.
 template <int KW, int KH, class Done>
-__device__ __forceinline__ void lg_l3_rows(const LegacyNet& N, int i, const float* __restrict__ in, int pitch, int last, f2_t nz, Done done) {
+__device__ __forceinline__ void lg_l3_rows(const LegacyNet& N, int i, const float* in, int pitch, int last, f2_t nz, Done done) {
     f2_t w[KH * KW];
 #pragma unroll
     for (int t = 0; t < KH * KW; ++t) w[t] = f2_pack(__ldg(&N.k3[2 * i][t]), __ldg(&N.k3[2 * i + 1][t]));
@@ -273,7 +273,7 @@ __device__ __forceinline__ void lg_l3_rows(const LegacyNet& N, int i, const floa
         const float* row = in + (size_t)min(r, last) * pitch;  // rows past the map feed responses past it
         f2_t v[KW];
 #pragma unroll
-        for (int c = 0; c < KW; ++c) v[c] = f2_dup(__ldg(row + c));
+        for (int c = 0; c < KW; ++c) v[c] = f2_dup(ld_chain(row + c));
 #pragma unroll
         for (int j = 0; j < kLgTY; ++j) {
             const int kr = r - j;
@@ -291,7 +291,7 @@ __device__ __forceinline__ void lg_l3_rows(const LegacyNet& N, int i, const floa
 // L3 to the output of one 32 x 8 tile of responses: a warp takes every eighth map pair for the whole tile,
 // then a thread a response sums what the pairs left in shared memory, in map (or neuron) order.
 template <int KW, int KH>
-__global__ void __launch_bounds__(kLgT) legacy_out_kernel(const LegacyNet* __restrict__ Np, const __grid_constant__ LgTable T, int* __restrict__ counts,
+__global__ void __launch_bounds__(kLgT) legacy_out_kernel(const LegacyNet* __restrict__ Np, const __grid_constant__ LgTable T, int* counts,
                                                           float thr, const f2_t nz) {
     __shared__ float vals[kLgMaxM2][kLgTY][kLgTX];  // L3 values, or without a fully connected layer each pair's sum
     chain_wait();
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kLgT) legacy_out_kernel(const LegacyNet* __res
             for (int j = 0; j < kLgTY && y0 + j < V.oh; ++j) {
                 f2_t acc = 0ull;
                 for (int t = 0; t < kt; ++t) {
-                    const f2_t m = f2_mul(f2_dup(__ldg(in + (size_t)(j + t / kw) * V.p2w + t % kw)), f2_pack(N.k3[2 * i][t], N.k3[2 * i + 1][t]), nz);
+                    const f2_t m = f2_mul(f2_dup(ld_chain(in + (size_t)(j + t / kw) * V.p2w + t % kw)), f2_pack(N.k3[2 * i][t], N.k3[2 * i + 1][t]), nz);
                     acc = t ? f2_add(acc, m) : m;
                 }
                 done(j, acc);

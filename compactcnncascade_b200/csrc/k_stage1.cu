@@ -57,7 +57,7 @@ struct FrontTile {
 // aligned with a pitch of whole float4 groups are read as 17 float4 per row (columns past the
 // image width hold zeros or the caller's own padding; no stored pixel depends on them), other
 // images one float at a time.
-__device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __restrict__ img, const LevelDesc& L, int ix0, int iy0) {
+__device__ __forceinline__ void load_front_tile(FrontTile& T, const float* img, const LevelDesc& L, int ix0, int iy0) {
     if (L.img_vec) {
         constexpr int kV = (kInW + 3) / 4;  // 17
         for (int i = threadIdx.x; i < kInH * kV; i += blockDim.x) {
@@ -66,7 +66,7 @@ __device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __res
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (y < L.h && x < L.img_pitch) {
                 const float4* src = reinterpret_cast<const float4*>(img + (long long)y * L.img_pitch + x);
-                v = __ldg(src);
+                v = *src;
             }
             T.put(r, 4 * c4, v.x);
             T.put(r, 4 * c4 + 1, v.y);
@@ -78,7 +78,7 @@ __device__ __forceinline__ void load_front_tile(FrontTile& T, const float* __res
             const int r = i / kInW, c = i - r * kInW;
             const int x = ix0 + c, y = iy0 + r;
             const float* src = img + (long long)y * L.img_pitch + x;
-            T.put(r, c, (x < L.w && y < L.h) ? (__ldg(src)) : 0.f);
+            T.put(r, c, (x < L.w && y < L.h) ? *src : 0.f);
         }
     }
 }
@@ -156,15 +156,15 @@ __device__ __forceinline__ ColRef col_ref(const GrayRef& G, const LevelDesc& L, 
 // Level pixels straight from the gray frame, resampled the way the pyramid kernel writes them (copy,
 // nearest neighbour, or bilinear on the 12-bit fixed-point steps; RunCPUDetect,
 // cnn_detector_v3.cpp:2090-2104, with ImageResizer, image_resize.cpp:46-122, 393-541), so the level image
-// is never stored. The gray frame was written by an earlier launch (read-only path). Samples past the
-// level's last row or column read the frame's own last ones: no stored pooled pixel depends on them.
+// is never stored. Samples past the level's last row or column read the frame's own last ones: no stored
+// pooled pixel depends on them.
 // kBilinear: (p0 * cx + p1 * fx) of the two gray rows as one packed chain, then top * cy + bot * fy.
 template <bool kBilinear>
 __device__ __forceinline__ float resample_px(const GrayRef& G, const RowRef& row, const ColRef& col, f2_t nz) {
     const float* p = G.p + (row.off + col.x);
-    if (!kBilinear) return __ldg(p);
+    if (!kBilinear) return *p;
     const float* q = p + G.pitch;
-    const f2_t l = f2_pack(__ldg(p), __ldg(q)), r = f2_pack(__ldg(p + 1), __ldg(q + 1));
+    const f2_t l = f2_pack(*p, *q), r = f2_pack(p[1], q[1]);
     const f2_t h = f2_mul(f2_add(f2_mul(l, col.c, nz), f2_mul(r, col.f, nz)), f2_ld(row.cf), nz);
     return fadd(f2_lo(h), f2_hi(h));
 }
@@ -243,8 +243,8 @@ __device__ __forceinline__ bool gate_live(const GateCells& cells, const LevelDes
 // back kernel computes exactly the live pixels' inputs, so a skipped strip is never read for a value that
 // is kept.
 template <bool kFromGray>
-__device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const LevelDesc& L, int t, const float* __restrict__ limg,
-                                           const GrayRef& G, float* __restrict__ s1, const GateCells& cells) {
+__device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const LevelDesc& L, int t, const float* limg,
+                                           const GrayRef& G, float* s1, const GateCells& cells) {
     constexpr int kWarps = kFrontThreads / 32;
     const int px0 = (t % L.k1_tiles_x) * kK1TileX;
     const int py0 = (t / L.k1_tiles_x) * kK1TileY;
@@ -359,9 +359,8 @@ __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const
 // stored level images limg (a caller's own level image)
 template <bool kFromGray, int kMinBlocks>
 __global__ void __launch_bounds__(kFrontThreads, kMinBlocks) stage1_front_kernel(const __grid_constant__ Stage1W W, const __grid_constant__ LevelTable LT,
-                                                              const float* __restrict__ limg, const GrayRef G, float* __restrict__ s1,
-                                                              const uint8_t* __restrict__ front_on, const GateCells cells, int* __restrict__ counts,
-                                                              int n_counts) {
+                                                              const float* limg, const GrayRef G, float* s1, const uint8_t* front_on,
+                                                              const GateCells cells, int* counts, int n_counts) {
     __shared__ FrontSmem S;
     chain_wait();
     if (blockIdx.x == 0)  // the back kernel's candidate counts start from zero
@@ -406,7 +405,7 @@ __device__ __forceinline__ void p2_unit(int p, int* x, int* y) {
 // columns past the plane pitch and rows past p1h are zero-filled (no valid response pixel depends on
 // them).
 template <int kThreads>
-__device__ __forceinline__ void load_back_map_async(BackSmem& S, const float* __restrict__ s1, const LevelDesc& L, int sx0, int sy0, int k) {
+__device__ __forceinline__ void load_back_map_async(BackSmem& S, const float* s1, const LevelDesc& L, int sx0, int sy0, int k) {
     const float* base = s1 + L.s1_off + (long long)k * L.s1_plane;
     constexpr int kV = kS1TW / 8;  // 16-byte vectors of a row's columns of one parity
     const int half = L.s1_pitch >> 1;
@@ -474,8 +473,8 @@ __device__ __forceinline__ f2_t pool_l2(const f2_t (*q)[4], const Stage1Back::L2
 // every pixel that is not live is written as the skip marker: only live pixels can become candidates,
 // and their inputs are exactly what runs (the front kernel skips the rest of S1).
 template <int kPairs, bool kCoherent>
-__device__ __forceinline__ void back_tile(const Stage1Back& D, BackSmem& S, const LevelDesc& L, int t, int g, const float* __restrict__ s1,
-                                          float* __restrict__ resp, int* __restrict__ counts, float thr, const uint8_t* __restrict__ back_on,
+__device__ __forceinline__ void back_tile(const Stage1Back& D, BackSmem& S, const LevelDesc& L, int t, int g, const float* s1,
+                                          float* resp, int* counts, float thr, const uint8_t* back_on,
                                           const GateCells& cells) {
     constexpr int kThreads = kK2TileX * kK2TileY / (2 * kPairs);
     constexpr int kWarps = kThreads / 32, kWarpRows = kK2TileY / kWarps;
@@ -658,8 +657,8 @@ __device__ __forceinline__ void back_tile(const Stage1Back& D, BackSmem& S, cons
 
 template <int kPairs, int kMinBlocks>
 __global__ void __launch_bounds__(256 / kPairs, kMinBlocks) stage1_back_kernel(const __grid_constant__ Stage1Back D, const __grid_constant__ LevelTable LT,
-                                                             const float* __restrict__ s1, float* __restrict__ resp, int* __restrict__ counts,
-                                                             float thr, const uint8_t* __restrict__ back_on, const GateCells cells) {
+                                                             const float* s1, float* resp, int* counts, float thr, const uint8_t* back_on,
+                                                             const GateCells cells) {
     __shared__ BackSmem S;
     const int g = LT.first + blockIdx.x;
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k2_base>(LT, g)];

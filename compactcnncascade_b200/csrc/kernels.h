@@ -16,7 +16,18 @@ namespace ccnn {
 // The kernels of a frame's chain are launched as programmatic dependents: a kernel's blocks are set up while
 // the one before it in the stream ends, and wait here, before they touch memory, until it has ended and its
 // writes are visible. Every block of such a kernel waits, so that the wait covers all earlier kernels too.
+// What an earlier kernel wrote is read by ordinary loads, never __ldg or a const __restrict__ pointer: those ask that
+// the data stay as they are while the kernel is resident, and the wait does not order them.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// An ordinary load of device memory that stays behind chain_wait (volatile keeps the two in order), for pointers read
+// from a table, whose space the compiler does not know: the legacy kernels took 25.5 and 19.6 us on B200 with generic
+// loads, 18.4 and 14.0 with these.
+__device__ __forceinline__ float ld_chain(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
 
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
