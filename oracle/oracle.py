@@ -82,9 +82,10 @@ def net_forward(stage, img, index_output):
     return out[: ow.value * oh.value].reshape(oh.value, ow.value)
 
 
-def detect(img, p=None, **kw):
+def detect(img, p=None, resp_cap=None, **kw):
     """Full detection with intermediates: gray, levels (w, h, scale), response maps, candidates,
-    raw detections (reference order) and final boxes."""
+    raw detections (reference order) and final boxes. resp_cap: response pixels of all levels (deep pyramids
+    need more than twice the frame's)."""
     p = p or params(**kw)
     L = load()
     h, w = img.shape[:2]
@@ -99,7 +100,7 @@ def detect(img, p=None, **kw):
     lh = np.empty(cap, np.int32)
     rw = np.empty(cap, np.int32)
     rh = np.empty(cap, np.int32)
-    resp = np.empty(2 * w * h + 1024, np.float32)  # upsampled pyramids hold more response pixels than the frame
+    resp = np.empty(resp_cap or 2 * w * h + 1024, np.float32)  # upsampled pyramids hold more response pixels than the frame
     ccap = w * h // 4 + 1024
     cands = (OrcCand * ccap)()
     nc = ctypes.c_int()
