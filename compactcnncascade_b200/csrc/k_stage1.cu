@@ -94,11 +94,10 @@ struct FrontStripRows {
     }
 };
 
-// Where a level row is sampled: the gray row's offset (floats) and, for bilinear levels, the row weights
-// (of the row and of the one below).
+// Where a level row is sampled: the gray row's offset (floats; 64 bits, a frame may have more than 2^32 pixels) and,
+// for bilinear levels, the row weights (of the row and of the one below).
 struct alignas(16) RowRef {
-    uint32_t off;
-    float pad;
+    size_t off;
     float2 cf;
 };
 
@@ -122,13 +121,13 @@ struct FrontSmem {
 __device__ __forceinline__ RowRef row_ref(const GrayRef& G, const LevelDesc& L, int y) {
     RowRef r{};
     if (L.mode == 0) {
-        r.off = (uint32_t)min(y, G.h - 1) * (uint32_t)G.pitch;
+        r.off = (size_t)min(y, G.h - 1) * G.pitch;
         return r;
     }
     const AxisSample sy = sample_row(y, L.scly, G.h);
     uint32_t py = sy.idx;
     if (L.mode == 2 && py + 1 >= (uint32_t)G.h) py--;  // bilinear keeps a row below
-    r.off = py * (uint32_t)G.pitch;
+    r.off = (size_t)py * G.pitch;
     r.cf = make_float2(sy.c, sy.f);
     return r;
 }
