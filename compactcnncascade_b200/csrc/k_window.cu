@@ -40,6 +40,8 @@ constexpr int kHalfW = kP1W / 2;      // 11: L1 pixels x and x + 11 of a row run
 constexpr int kP1Pairs = kHalfW * kP1H;
 constexpr int kInPairs = 2 * kHalfW + 3;  // 25 columns of a row of input pairs
 
+constexpr int kMaxRest = 16;  // L1 pairs (CNTK) or pixels (legacy) past the whole passes
+
 struct WindowSmem {
     uint8_t crop[kCropH][kCropW + 3];
     int hist[256];
@@ -60,10 +62,13 @@ struct WindowSmem {
         float hbuf[84][kOutN];          // after L3
     } v;
     float out[kOutN];
-    float2 l1rest[32][6];  // pooled L1 maps of the partial pass's pixels
+    float2 l1rest[kMaxRest][6];  // pooled L1 maps of the partial pass's pixels
     int geo[4];
 };
 static_assert(kInPairs <= 30, "columns of an input row");
+// six resident blocks a SM (a schedule knob's value): 228 KB, of which each block also takes its static 32 bytes and
+// 1 KB, in steps of 128 bytes
+static_assert(6 * ((sizeof(WindowSmem) + 32 + 1024 + 127) / 128 * 128) <= 228 * 1024, "six blocks a SM");
 
 // mode: 0 = stage-2 view (columns 2..48), 1 = mirrored (46 - x), 2 = plain (columns 0..46)
 __device__ __forceinline__ float win_in(const WindowSmem& S, int mode, int x, int y) {
@@ -95,7 +100,7 @@ __device__ void window_net(const NW& W, const NW* __restrict__ G, WindowSmem& S,
     // once. 256 pairs take a pass of every map a thread; the last 8 are split into (pair, map) units, one
     // warp a map, so that they take a sixth of a pass.
     constexpr int kRest = kP1Pairs - kWT;
-    static_assert(kRest > 0 && kRest <= 32 && NW::kM1 <= kWT / 32, "one full pass, the rest a warp a map");
+    static_assert(kRest > 0 && kRest <= kMaxRest && NW::kM1 <= kWT / 32, "one full pass, the rest a warp a map");
     auto pooled = [&](const f2_t (&win)[5][5], int m) {
         f2_t c[4];
 #pragma unroll
@@ -242,7 +247,7 @@ __device__ void legacy_window_net(const LegacyNet& W, WindowSmem& S, int mode, f
     constexpr int kP2 = kP2W * kP2H;
     constexpr int kM0 = 6;  // the most first-layer maps of a stage-2/3 network
     constexpr int kFull = (kP1W * kP1H / kWT) * kWT, kRest = kP1W * kP1H - kFull, kMP = kM0 / 2;
-    static_assert(kRest > 0 && kRest <= 32 && 32 * kMP <= kWT, "partial L1 pass must fit one warp per map pair");
+    static_assert(kRest > 0 && kRest <= kMaxRest && 32 * kMP <= kWT, "partial L1 pass must fit one warp per map pair");
     const int m0 = W.m0;
     const f2_t af = f2_dup(W.af);
     auto sums = [&](const float (&P)[kM0], int px) {
