@@ -457,7 +457,8 @@ __device__ __forceinline__ f2_t pool_l2(const f2_t (*q)[4], const Stage1Back::L2
 // back: one CTA per 32 x 16 tile of response pixels, every operation packed over the pixels (x, x + 16)
 // of a row, so that no operand has to be duplicated or paired in registers. kPairs pixel pairs a thread
 // in C (256 / kPairs threads): two halve the constant loads a pixel, which share one queue with the
-// shared-memory loads, and suit launches with many tiles a SM; one gives a tile twice the warps.
+// shared-memory loads, and suit launches with many tiles a SM; one gives a tile twice the warps
+// (back_pixel_pairs).
 // The four S1 maps of the tile (42 x 72 each) pass through shared memory one after the other; for map k
 //   A: the pooled L2 maps 2k and 2k + 1 on the 35 x 20 halo tile, and the neighbour sums whose three maps
 //      are now known (the two partial sums a pixel still needs stay in registers);
@@ -737,18 +738,14 @@ cudaError_t launch_stage1_back(const Stage1W& W, const LevelDesc* levels, int n_
                                int* counts, float thr, const uint8_t* back_on, GateCells cells, Stage1Sched sched) {
     const Stage1Back D = make_back(W);
     if (n_levels <= 0) return cudaSuccess;
-    // Two pixel pairs a thread do the same work with 8 % fewer instructions, but a tile then has 4 warps
-    // instead of 8 and takes longer by itself. They are used where every SM has at least two tiles to run
-    // (3840x2160, scale 1.05: 1.34 ms a frame against 1.72; 1080p: 53 us against 61); below that, and
-    // with the learned gate, which runs about a quarter of the tiles and skips by warps of 32 x 2 pixels
-    // instead of 32 x 4, one pair (640x480: 27.6 us against 29.6; a gated 1080p frame 37 us against 43).
-    constexpr int kTwoPairTiles = 296;
-    const LevelDesc& last = levels[n_levels - 1];
-    const int tiles = last.k2_base + last.k2_tiles_x * ((last.oh + kK2TileY - 1) / kK2TileY);
-    const bool two_pairs = tiles >= kTwoPairTiles && !back_on;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     return launch_grouped(
         levels, n_levels, &LevelDesc::k2_base, [](const LevelDesc& L) { return L.k2_tiles_x * ((L.oh + kK2TileY - 1) / kK2TileY); },
         [&](const LevelTable& T, int blocks) {
+            const bool two_pairs = back_pixel_pairs(blocks, sms, back_on != nullptr) == 2;
             const auto kernel = two_pairs ? (sched.back_blocks_per_sm >= 4 ? stage1_back_kernel<2, 6> : stage1_back_kernel<2, 5>) : stage1_back_kernel<1, 3>;
             return launch_chained(kernel, blocks, two_pairs ? 128 : 256, 0, st, D, T, s1, resp, counts, thr, back_on, cells);
         });

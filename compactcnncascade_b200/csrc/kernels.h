@@ -207,6 +207,15 @@ struct Stage1Sched {
     int front_blocks_per_sm = 3;
     int back_blocks_per_sm = 4;
 };
+// Pixel pairs a thread of a back launch of `tiles` tiles on `sms` SMs. Two do the same work with 8 % fewer
+// instructions, but a tile then has 4 warps instead of 8 and takes longer by itself. They are used where every SM
+// has at least two tiles to run (3840x2160, scale 1.05: 1.34 ms a frame against 1.72; 1080p: 53 us against 61);
+// below that, and with the learned gate, which runs about a quarter of the tiles and skips by warps of 32 x 2 pixels
+// instead of 32 x 4, one (640x480: 27.6 us against 29.6; the last 44 tiles of the 3840x2160 frame's third launch 21.5
+// against 26.0; a gated 1080p frame 37 us against 43). The one-pair kernel
+// has a single build, so back_blocks_per_sm does not reach it. The persistent kernel, whose blocks take front tiles
+// too, always runs two.
+inline int back_pixel_pairs(int tiles, int sms, bool gated) { return tiles >= 2 * sms && !gated ? 2 : 1; }
 // the frame's gray image as the stage-1 front kernel resamples each level tile from it; p == nullptr:
 // the level images are stored (limg + img_off) and read instead
 struct GrayRef {
