@@ -236,7 +236,8 @@ __device__ __forceinline__ bool gate_live(const GateCells& cells, const LevelDes
 // from the stored level images limg by the block), then the 4x4 conv + folded BN/LReLU + 2x2 max of the 4
 // L1 maps for 32 x 16 pooled pixels, a warp a strip of 2 x 32 (two vertically adjacent pixels a thread), and
 // the 4 neighbour-map sums written to the S1 arena.
-// cells (the learned gate, optional): a strip that feeds no live response pixel is not computed. S1 row y
+// cells (the learned gate, optional; frames only, a stored image is always computed in full): a strip that feeds no
+// live response pixel is not computed. S1 row y
 // feeds pooled-L2 rows ceil((y - 3) / 2) .. y / 2 (a 3x3 conv at the 2x2 pool positions), and L2 row Y
 // feeds response rows Y - 4 .. Y (the 4-wide, 5-tall L3 kernel); columns alike with the 4-wide kernel. The
 // back kernel computes exactly the live pixels' inputs, so a skipped strip is never read for a value that
@@ -326,7 +327,6 @@ __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const
         }
         return;
     }
-    uint32_t live = (1u << strips) - 1u;
     if (kFromGray) {
         // the full scan: the block resamples the tile once
         if (threadIdx.x < kInH) S.rows[threadIdx.x] = row_ref(G, L, iy0 + threadIdx.x);
@@ -337,20 +337,11 @@ __device__ __forceinline__ void front_tile(const Stage1W& W, FrontSmem& S, const
         else
             resample_front_tile<false>(S, G, L, ix0, rows, nz);
     } else {
-        if (gate_gating(cells)) {
-            __shared__ int s_flive[kStrips];
-            if (threadIdx.x < kStrips) s_flive[threadIdx.x] = strip_live(threadIdx.x) ? 1 : 0;
-            __syncthreads();
-#pragma unroll
-            for (int s = 0; s < kStrips; ++s)
-                if (!s_flive[s]) live &= ~(1u << s);
-        }
         load_front_tile(S.T, limg + L.img_off, L, ix0, iy0);
     }
     __syncthreads();
 #pragma unroll 1
-    for (int s = warp; s < strips; s += kWarps)
-        if ((live >> s) & 1u) strip(s, &S.T.p[4 * s]);  // a strip without a live pixel downstream writes nothing
+    for (int s = warp; s < strips; s += kWarps) strip(s, &S.T.p[4 * s]);
 }
 
 
@@ -466,13 +457,14 @@ __device__ __forceinline__ f2_t pool_l2(const f2_t (*q)[4], const Stage1Back::L2
 //      part of the output sum, all in registers, while S1 map k + 1 is copied (cp.async).
 // Two S1 maps and three sums are ever held, 33 KB, so that registers alone limit the resident blocks.
 // Back tile t of level L as above; g is its global back-tile index (the gate's tile index).
-// kCoherent: the S1 arena was written earlier in the same launch (read through L2).
+// The S1 arena may have been written earlier in the same launch (the persistent kernel): its copies go through L2
+// (cp.async.cg), where those writes are.
 // Warps (32 x 2 kPairs response pixels) and L2 rows that only pixels past the map's last row need are
 // skipped. With the learned gate (cells), a warp without a live pixel writes the skip marker instead of
 // computing, A computes only the rows live warps read (a warp's rows and the four after them), and
 // every pixel that is not live is written as the skip marker: only live pixels can become candidates,
 // and their inputs are exactly what runs (the front kernel skips the rest of S1).
-template <int kPairs, bool kCoherent>
+template <int kPairs>
 __device__ __forceinline__ void back_tile(const Stage1Back& D, BackSmem& S, const LevelDesc& L, int t, int g, const float* s1,
                                           float* resp, int* counts, float thr, const uint8_t* back_on,
                                           const GateCells& cells) {
@@ -664,7 +656,7 @@ __global__ void __launch_bounds__(256 / kPairs, kMinBlocks) stage1_back_kernel(c
     const LevelDesc& L = LT.lv[find_level<&LevelDesc::k2_base>(LT, g)];
     const int t = g - L.k2_base;
     chain_wait();
-    back_tile<kPairs, false>(D, S, L, t, g, s1, resp, counts, thr, back_on, cells);
+    back_tile<kPairs>(D, S, L, t, g, s1, resp, counts, thr, back_on, cells);
 }
 
 // The back kernel's parameters, derived from the packed weight block.
@@ -862,7 +854,7 @@ __global__ void __launch_bounds__(kBatchThreads, 5) stage1_batch_kernel(const __
                 front_tile<true>(W, *reinterpret_cast<FrontSmem*>(smem_raw), L, g - L.k1_base, nullptr,
                                         GrayRef{F.gray[f], F.gpitch, F.gw, F.gh}, F.s1[f], F.cells[f]);
         } else {
-            back_tile<2, true>(D, *reinterpret_cast<BackSmem*>(smem_raw), L, g - L.k2_base, g, F.s1[f], F.resp[f], F.counts[f], Q.thr,
+            back_tile<2>(D, *reinterpret_cast<BackSmem*>(smem_raw), L, g - L.k2_base, g, F.s1[f], F.resp[f], F.counts[f], Q.thr,
                             F.back_on[f], F.cells[f]);
         }
         __syncthreads();  // every thread is done with the item (and with the shared memory)

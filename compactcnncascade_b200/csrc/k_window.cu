@@ -238,8 +238,8 @@ __device__ void window_net(const NW& W, const NW* __restrict__ G, WindowSmem& S,
 }
 
 // The legacy (format 1.0) stage-2/3 networks on the window in shared memory: the sums of neighbouring L1 maps
-// (6 maps, 22x24 pooled) in S.s1, L2 (12 maps, 10x11) in S.p2 and their sums in S.s2, the L3 values of the
-// 16 outputs in S.a3, fully connected hidden neurons in S.hbuf; the arithmetic of the standalone legacy
+// (6 maps, 22x24 pooled) in S.s1, L2 (12 maps, 10x11) in S.u.l.p2 and their sums in S.u.l.s2, the L3 values of the
+// 16 outputs in S.u.l.a3, fully connected hidden neurons in S.v.hbuf; the arithmetic of the standalone legacy
 // forward pass (legacy_dev.cuh), map pairs packed, spread over the block. As in window_net, whole passes of
 // L1 pixels take every map pair a thread and the pixels of the last, partial pass one pair a warp. The windows
 // of a 640 x 480 frame took 81 us on B200 with one map a thread and the map sums made tap by tap, now 40.
