@@ -8,15 +8,17 @@ The knobs (include/ccnn_inspect.h, ccnn_schedule):
   window_ctas_per_sm   resident blocks per SM of the persistent stage-2/3 window kernel (5, 6: builds
                        with 48 and 40 registers a thread)
   front_blocks_per_sm  register budget of the stage-1 front kernel (3: 5 blocks of 128 threads a SM, 4: 6)
-  back_blocks_per_sm   register budget of the stage-1 back kernel (3: 5 blocks of 128 threads a SM, 4: 6)
+  back_blocks_per_sm   register budget of the stage-1 back kernel (3: 5 blocks of 128 threads a SM, 4: 6); no
+                       effect with the gate on or where a launch has fewer than two tiles a SM (one build)
   batch_frames         frames per batched graph (0: every frame its own graph; 1: the same with the
                        pyramid and stage 1 of all levels in one persistent launch); the batched form
                        runs the pyramid and stage 1 of a whole group in one persistent launch
   batch_blocks_per_sm  how much of a SM that persistent kernel fills (its grid: twice this many blocks of 128
-                       threads a SM, at most the 5 that fit; fewer leave SMs to other frames' kernels)
+                       threads a SM, at most the 5 that fit, so 3 and 4 are the same; fewer leave SMs to
+                       other frames' kernels)
 
 The search is coordinate descent from the defaults: each knob in turn takes the value that times
-fastest with the others held, for two passes (a full product of the knobs would be 960 timings).
+fastest with the others held, for two passes (a full product of the knobs would be 1,800 timings).
 
     python -m compactcnncascade_b200.autotune --width 1920 --height 1080 [--gate]
 """
@@ -30,7 +32,7 @@ from . import _capi
 
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "schedules.json")
 KNOBS = (("frame_slots", (4, 8, 12, 16, 24, 32)), ("window_ctas_per_sm", (2, 3, 4, 5, 6)), ("front_blocks_per_sm", (3, 4)),
-         ("back_blocks_per_sm", (3, 4)), ("batch_frames", (0, 1, 2, 4, 8)), ("batch_blocks_per_sm", (1, 2, 3, 4)))
+         ("back_blocks_per_sm", (3, 4)), ("batch_frames", (0, 1, 2, 4, 8)), ("batch_blocks_per_sm", (1, 2, 3)))
 DEFAULTS = {"frame_slots": 8, "window_ctas_per_sm": 4, "front_blocks_per_sm": 3, "back_blocks_per_sm": 4, "batch_frames": 0,
             "batch_blocks_per_sm": 3}
 

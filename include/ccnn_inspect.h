@@ -124,13 +124,14 @@ CCNN_API ccnn_status ccnn_set_schedule(ccnn_handle h, int frame_slots, int windo
 CCNN_API ccnn_status ccnn_get_schedule(ccnn_handle h, int* frame_slots, int* window_ctas_per_sm);
 
 /* The full schedule: the two knobs above, the register budget of the two stage-1 kernels
- * (3 or 4: more resident blocks hide more latency, fewer registers may spill), and the batched form:
+ * (3 or 4: more resident blocks hide more latency, fewer registers may spill; the back kernel has one build
+ * with the learned gate on and where a launch has fewer than two tiles a SM), and the batched form:
  * batch_frames > 1 runs groups of that many frames of one size through ccnn_detect_batch / ccnn_detect_device_batch as one graph each (the pyramid and stage 1
  * of every level of every frame of the group in one persistent launch fed by a device work queue,
  * then the candidates, windows and replays of the group in one launch each); frame_slots must be at
  * least batch_frames, and frame_slots / batch_frames groups are in flight. batch_blocks_per_sm (1-4)
  * is how much of a SM the persistent kernel fills (its grid: twice that many blocks of 128 threads a SM, at
- * most what fits; fewer blocks leave SMs to other frames' kernels). 0 keeps a value
+ * most the 5 that fit, so 3 and 4 are the same; fewer blocks leave SMs to other frames' kernels). 0 keeps a value
  * (batch_frames: -1 keeps it, 0 turns the batched form off). Same rules as ccnn_set_schedule. */
 typedef struct {
     int frame_slots;
