@@ -7,9 +7,9 @@
 // where it is needed (72 of a pixel's 1,872 multiply-adds, against 64 bytes of traffic a pixel). Both
 // are persistent, a block of 128 threads a tile of 32 x 16 pixels at a time with its halo in shared
 // memory, and keep their gradient sums in registers over all their tiles, so there are no atomics and
-// every run gives the same bits. A step on 64 frames of 240 x 135 takes 0.26 ms on B200 (3.1 ms when every
-// map passed through memory, a weight gradient was one thread's walk over the pixels of a row band and
-// the sums were atomics): 3.9 G multiply-adds, 0.11 ms at the fp32 pipe's rate.
+// every run gives the same bits. A step on 64 frames of 240 x 135 takes 0.28 ms on B200: 0.1 forward, 0.17
+// backward, 0.009 update (3.1 ms when every map passed through memory, a weight gradient was one thread's walk
+// over the pixels of a row band and the sums were atomics): 3.9 G multiply-adds, 0.11 ms at the fp32 pipe's rate.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -182,7 +182,7 @@ struct ForwardSmem {
 // Forward pass, loss, the head's gradients (part[block][kHeadGrads + 1], the loss last), and per pooled
 // cell the gradient of its 8 averages (gq) and per pixel the signs of a2 (a bit a map). A lane pair's
 // 2 x 4 pixels are two cells, one a lane.
-// Bound by the fp32 pipe (652 multiply-adds a pixel, 56 % busy) and the latency between its barriers: 0.1 ms
+// Bound by the fp32 pipe (652 multiply-adds a pixel, 58 % busy) and the latency between its barriers: 0.1 ms
 // for 64 frames of 240 x 135.
 __global__ void __launch_bounds__(kTT, 4) gate_forward_kernel(const float* __restrict__ P, const __half* __restrict__ feat,
                                                               const uint8_t* __restrict__ labels, const TrainShape s, float pos_weight,
@@ -361,8 +361,8 @@ __device__ __forceinline__ void load_gz2(float* g, float* sum, const float4* __r
 // The convolutions' gradients (part[block][kConvGrads]) from gz2: W2's (8 x 8 x 9 sums of gz2 x a1 over the
 // pixels), gz1 by the transposed convolution, and W1's (8 x 9 sums of gz1 x f). For W2's a lane holds
 // the 72 sums of one input map (lane % 8) over the rows lane / 8 of its warp's four; for W1's the 9 of one
-// map. Bound by the fp32 pipe (1,296 multiply-adds a pixel, 56 % busy) and its five barriers a tile, with
-// three blocks a SM (the 72 + 9 sums a thread): 0.165 ms for 64 frames of 240 x 135.
+// map. Bound by the fp32 pipe (1,296 multiply-adds a pixel, 58 % busy) and its five barriers a tile, with
+// three blocks a SM (the 72 + 9 sums a thread): 0.17 ms for 64 frames of 240 x 135.
 __global__ void __launch_bounds__(kTT, 3) gate_backward_kernel(const float* __restrict__ P, const __half* __restrict__ feat,
                                                                const float4* __restrict__ gq, const uint8_t* __restrict__ signs,
                                                                const TrainShape s, float* __restrict__ part) {

@@ -10,18 +10,18 @@
 //        read instead where the caller gives one; with the learned gate each warp resamples only the 7
 //        rows of a strip of two pooled rows and runs on its own), runs the 4x4 conv + folded
 //        BN/LReLU + 2x2 max for the 4 L1 maps and writes the 4 neighbour-map sums that L2 consumes
-//        (S1 arena). Bound by the fp32 pipe (65 % busy; about 87 % is what these packed chains reach
-//        alone) and the latency of the gray samples: 1.09 ms for the 83 levels of a 3840x2160 frame at
-//        scale 1.05 (1.30 with 256-thread blocks and 25 % more instructions: the row references once a tile
-//        instead of once a sample, both gray rows of a sample as one packed chain), 39.8 us for the 13 of a
-//        1080p frame (43.3); two weights a constant load instead of one took 3 % more off.
+//        (S1 arena). Bound by the fp32 pipe (65 % busy with every SM full; independent chains of these packed
+//        instructions alone reach 96 %, k_peak.cu) and the latency of the gray samples: 1.07 ms for the 83 levels
+//        of a 3840x2160 frame at scale 1.05 (1.30 with 256-thread blocks and 25 % more instructions: the row
+//        references once a tile instead of once a sample, both gray rows of a sample as one packed chain, two weights
+//        a constant load), 36 us for the 13 of a 1080p frame (43.3).
 // back:  one CTA per 32x16 tile of response pixels (128 threads with two pixel pairs a thread, 256 with
 //        one). It takes the S1 tile (4 x 42 x 72) map by map through two shared-memory buffers
 //        (asynchronous copies), computes the pooled L2 maps of each and the sums they complete on the
 //        35 x 20 halo tile, then the 16 L3 maps (4w x 5h), the 52 hidden neurons and the output sum as far
-//        as those reach. Bound by the fp32 pipe (65 % busy): 1.35 ms for the 83 levels (1.64 when a thread
-//        packed two vertical neighbours, whose operands had to be paired in registers, with two
-//        reciprocal steps and twice the constant loads a pixel), 53 us for the 13 (61).
+//        as those reach. Bound by the fp32 pipe (69 % busy with every SM full): 1.36 ms for the 83 levels (1.64 when a
+//        thread packed two vertical neighbours, whose operands had to be paired in registers, with two
+//        reciprocal steps and twice the constant loads a pixel), 49 us for the 13 (58).
 // Both kernels come in two register budgets, chosen per workload by the schedule (Stage1Sched).
 // Packed f32x2 instructions run two identical chains of IEEE operations at once (two pixels, or
 // two maps that read the same input), so every value still sees the reference's roundings.
